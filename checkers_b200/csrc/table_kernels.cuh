@@ -9,14 +9,10 @@
 //
 // The reference hands out (or takes back) rounding slots in the order
 // std::sort leaves the symbols in when sorted by the fractional part of their
-// ideal share.  When slots are handed out only the SET of the first `rem`
-// symbols matters, and that set does not depend on the order of equal
-// fractions unless a group of equal fractions straddles position `rem`: each
-// thread counts the fractions above and not below its own and decides for
-// itself.  Only the straddling case, and the case where slots are taken back
-// (which walks the order from its end, skipping symbols that hold one slot),
-// need the order itself; one thread then runs sort_replica -- the library's
-// algorithm restated move for move -- and applies the reference's loops.
+// ideal share, and std::sort is not stable: where fractions are equal the order
+// is whatever the library's algorithm leaves behind.  sort_replica.hpp restates
+// that algorithm move for move; here the same moves are made by the 256 threads
+// of the table's CTA together (block_sort_order).
 #pragma once
 #include "sort_replica.hpp"
 
@@ -35,12 +31,11 @@ struct TableJob {
 
 struct NormSmem {
     FracKey keys[256];
-    double frac[256];
-    uint32_t slots[256];
+    uint32_t mask_a[8], mask_b[8];
+    uint16_t pos_a[256], pos_b[256], cut[256];
+    uint16_t place[256];  // by symbol: its position in the sorted order
     uint32_t warp_a[8], warp_b[8];
     unsigned long long warp_c[8];
-    uint32_t n_keys, assigned, need_sort;
-    unsigned long long total;
 };
 
 // Sums over the 256 threads of a CTA (all threads get the result).
@@ -86,6 +81,83 @@ __device__ __forceinline__ uint32_t block_scan256(uint32_t v, uint32_t* warp_par
     }
     *total_out = total;
     return before + inc - v;
+}
+
+// Set bits of a 256-bit mask in [lo, hi).
+__device__ __forceinline__ uint32_t mask_count(const uint32_t* mask, uint32_t lo, uint32_t hi) {
+    uint32_t c = 0;
+    for (uint32_t w = lo >> 5; w * 32 < hi; ++w) {
+        uint32_t m = mask[w];
+        if (w * 32 < lo) m &= 0xFFFFFFFFu << (lo & 31);
+        if (hi < w * 32 + 32) m &= ~(0xFFFFFFFFu << (hi & 31));
+        c += (uint32_t)__popc(m);
+    }
+    return c;
+}
+
+// keys[0..n) sorted as sort_replica sorts them; sm.place[symbol] receives the positions.
+// One thread walking the introsort took about 100 us a table; almost all of it is the Hoare partitions, and those
+// can be done at once.  A partition of [F + 1, L) about p swaps the k-th element from the left that does not stand
+// before p with the k-th from the right that p does not stand before, for as long as the first lies left of the
+// second: thread i finds the rank of its element among either kind by counting bits, and the pairs are disjoint.
+// With K swaps made, the next left stop (or, if that is further right, the last element swapped to the right, which
+// now stops the scan) is the cut.  Ranges of one recursion level are independent and run side by side, all at
+// the same depth; the final insertion sort never moves an element past an equal one, so it is a stable sort of
+// what the partitions leave, and an element only moves inside its range of 16 or fewer.
+__device__ __forceinline__ void block_sort_order(NormSmem& sm, uint32_t n) {
+    const uint32_t i = threadIdx.x, warp = i >> 5, lane = i & 31;
+    uint32_t F = 0, L = n, depth = 0;  // this position's range
+    while ((2u << depth) <= n) ++depth;
+    depth *= 2;  // 2 * floor(log2 n)
+    for (;; --depth) {
+        const bool active = i < n && L - F > 16;
+        if (block_sum256(active ? 1u : 0u, sm.warp_a) == 0) break;
+        if (depth == 0) {
+            if (active && i == F) sr_heap_sort(sm.keys + F, sm.keys + L);
+            __syncthreads();
+            break;
+        }
+        if (active && i == F) sr_median_to_first(sm.keys + F, sm.keys + F + 1, sm.keys + F + (L - F) / 2, sm.keys + L - 1);
+        __syncthreads();
+        const double p = active ? sm.keys[F].frac : 0.0, v = active ? sm.keys[i].frac : 0.0;
+        const bool a = active && i > F && !(v > p), b = active && i > F && !(p > v);
+        const uint32_t ma = __ballot_sync(0xffffffffu, a), mb = __ballot_sync(0xffffffffu, b);
+        if (lane == 0) {
+            sm.mask_a[warp] = ma;
+            sm.mask_b[warp] = mb;
+        }
+        __syncthreads();
+        const uint32_t ra = a ? mask_count(sm.mask_a, F + 1, i) : 0u;
+        if (a) sm.pos_a[F + ra] = (uint16_t)i;
+        if (b) sm.pos_b[F + mask_count(sm.mask_b, i + 1, L)] = (uint16_t)i;
+        __syncthreads();
+        if (a) {
+            const uint32_t na = mask_count(sm.mask_a, F + 1, L), nb = mask_count(sm.mask_b, F + 1, L);
+            const uint32_t mate = ra < nb ? sm.pos_b[F + ra] : 0u;  // 0: none (a position right of F is never below it)
+            if (i < mate) {
+                const uint32_t next = ra + 1 < na ? sm.pos_a[F + ra + 1] : 0xFFFFu;
+                if (!(ra + 1 < nb && next < sm.pos_b[F + ra + 1])) sm.cut[F] = (uint16_t)(next < mate ? next : mate);
+                sr_swap(sm.keys[i], sm.keys[mate]);
+            } else if (ra == 0) {
+                sm.cut[F] = (uint16_t)i;
+            }
+        }
+        __syncthreads();
+        if (active) {
+            const uint32_t c = sm.cut[F];
+            if (i < c) L = c; else F = c;
+        }
+    }
+    if (i < n) {
+        const double v = sm.keys[i].frac;
+        uint32_t at = F;
+        for (uint32_t k = F; k < L; ++k) {
+            const double o = sm.keys[k].frac;
+            at += o > v || (o == v && k < i);
+        }
+        sm.place[sm.keys[i].sym] = (uint16_t)at;
+    }
+    __syncthreads();
 }
 
 // The encode entry of one symbol (same arithmetic as build_enc_entries in tables.hpp).
@@ -143,33 +215,12 @@ __global__ void __launch_bounds__(256) normalize_tables_kernel(const TableJob* _
             const double fr = exact - (double)(int)exact;
             const uint32_t assigned = block_sum256(slot, sm.warp_a);
             const uint32_t n_keys = block_sum256(present ? 1u : 0u, sm.warp_b);
-            bool need_sort = assigned > kM;
-            if (assigned < kM) {
-                const uint32_t rem = kM - assigned;
-                if (rem >= n_keys) {
-                    slot += present ? 1u : 0u;
-                } else {
-                    __syncthreads();
-                    sm.frac[s] = present ? fr : -1.0;  // real fractions are never negative
-                    __syncthreads();
-                    uint32_t greater = 0, not_less = 0;
-                    for (uint32_t k = 0; k < 256; ++k) {
-                        const double o = sm.frac[k];
-                        greater += o > fr;
-                        not_less += o >= fr;
-                    }
-                    const bool in = present && not_less <= rem;    // among the first rem whatever the tie order
-                    const bool out = !present || greater >= rem;   // behind them whatever the tie order
-                    need_sort = block_sum256((!in && !out) ? 1u : 0u, sm.warp_a) != 0;
-                    if (!need_sort) slot += in ? 1u : 0u;
-                }
-            }
-            if (need_sort) {
+            if (assigned < kM && kM - assigned >= n_keys) {
+                slot += present ? 1u : 0u;
+            } else if (assigned != kM) {
                 // keys in symbol order, exactly the vector the reference sorts
                 uint32_t n_tot;
                 const uint32_t pos = block_scan256(present ? 1u : 0u, sm.warp_a, &n_tot);
-                __syncthreads();
-                sm.slots[s] = slot;
                 if (present) {
                     FracKey key;
                     key.frac = fr;
@@ -178,26 +229,26 @@ __global__ void __launch_bounds__(256) normalize_tables_kernel(const TableJob* _
                     sm.keys[pos] = key;
                 }
                 __syncthreads();
-                if (s == 0) {
-                    sort_replica(sm.keys, (int)n_tot);
-                    if (assigned < kM) {
-                        uint32_t rem = kM - assigned;
-                        for (uint32_t k = 0; k < n_tot && rem; ++k, --rem) sm.slots[sm.keys[k].sym]++;
-                    } else {
-                        uint32_t rem = assigned - kM;
-                        for (;;) {
-                            const uint32_t before = rem;
-                            for (int k = (int)n_tot - 1; k >= 0 && rem; --k)
-                                if (sm.slots[sm.keys[k].sym] > 1) {
-                                    sm.slots[sm.keys[k].sym]--;
-                                    --rem;
-                                }
-                            if (!(job.flags & kTableRepair) || rem == 0 || rem == before) break;
-                        }
+                block_sort_order(sm, n_tot);
+                const uint32_t at = present ? sm.place[s] : 0u;
+                if (assigned < kM) {
+                    slot += present && at < kM - assigned ? 1u : 0u;
+                } else {
+                    // slots are taken back from the end of the order, one per symbol that has more than one
+                    uint32_t rem = assigned - kM;
+                    for (;;) {
+                        if (s < 8) sm.mask_a[s] = 0;
+                        __syncthreads();
+                        const bool can = present && slot > 1;
+                        if (can) atomicOr(&sm.mask_a[at >> 5], 1u << (at & 31));
+                        __syncthreads();
+                        if (can && mask_count(sm.mask_a, at + 1, n_tot) < rem) --slot;
+                        const uint32_t before = rem, able = mask_count(sm.mask_a, 0, n_tot);
+                        rem -= able < rem ? able : rem;
+                        __syncthreads();
+                        if (!(job.flags & kTableRepair) || rem == 0 || rem == before) break;
                     }
                 }
-                __syncthreads();
-                slot = sm.slots[s];
             }
         }
         uint32_t sum;
