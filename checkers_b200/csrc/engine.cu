@@ -132,8 +132,8 @@ struct Context {
     bool decode_zero_skip = false; // float tensors whose table allows it are decoded with the short slot table (measured slower)
 
     // device buffers (grow-only, from the context's pool)
-    DevBuf d_descs, d_tiles, d_hist, d_sidecar, d_scratch, d_hdrs, d_order, d_ticket, d_psize, d_zslots, d_zregions, d_zslot_of, d_jobs, d_sums, d_stats_part, d_stats_mid, d_poff, d_fileorder, d_hll32, d_hll8, d_symkeys, d_symcounts,
-        d_payload, d_enc, d_freq, d_cum, d_status, d_stats_desc, d_stats_out;
+    DevBuf d_descs, d_tiles, d_hist, d_sidecar, d_scratch, d_hdrs, d_order, d_ticket, d_psize, d_zslots, d_zregions, d_zslot_of, d_jobs, d_sums, d_stats_part, d_stats_mid, d_poff, d_fileorder, d_lane_src, d_lane_off, d_items, d_hll32, d_hll8, d_symkeys, d_symcounts,
+        d_payload, d_enc, d_freq, d_cum, d_stats_desc, d_stats_out;
     cudaStream_t side_stream = nullptr;
     std::vector<cudaEvent_t> ev_count, ev_tab;
     int segments = 4;             // launches the counting of a batch is cut into (tables of a piece are built under the next)
@@ -141,8 +141,9 @@ struct Context {
     int encode_teams_per_sm = 0;  // cap on resident encode teams per SM and launch (0 = as many as fit)
     int decode_teams_per_sm = 0;  // same for the decode grid
     int sm_count = 0;
+    std::unordered_map<const void*, int> resident_teams;  // per SM, of each persistent kernel this context has launched
     // pinned host staging
-    PinBuf h_hdrs, h_poff, h_psize, h_descs, h_status, h_jobs, h_sums, h_freq, h_cum, h_stats, h_order, h_tiles;
+    PinBuf h_hdrs, h_poff, h_psize, h_descs, h_status, h_jobs, h_sums, h_freq, h_cum, h_stats, h_order, h_tiles, h_items;
     PinBuf img[3];  // states, mantissa, tables
     // Where the next compress builds its file images instead of img[] (caller-owned pinned memory of
     // at least the worst-case sizes); the chunked host pipeline keeps one set per part this way.
@@ -222,9 +223,32 @@ __global__ void control_copy_kernel(uint32_t* __restrict__ dst, const uint32_t* 
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += (size_t)gridDim.x * blockDim.x)
         dst[i] = src[i];
 }
-__global__ void control_fill_kernel(uint32_t* __restrict__ dst, size_t n_words) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += (size_t)gridDim.x * blockDim.x)
-        dst[i] = 0u;
+// Several such copies, or fills with zero (src null), in one launch: what a call uploads before its first kernel and
+// what it brings back after its last is a handful of small arrays, and a launch each cost more than the copies.
+struct ControlOps {
+    static constexpr int kMax = 8;
+    struct Op {
+        uint32_t* dst;
+        const uint32_t* src;
+        size_t words;
+    } op[kMax];
+    int n = 0;
+    size_t words = 0;  // the longest op
+    void copy(void* dst, const void* src, size_t bytes) {
+        if (bytes == 0) return;
+        op[n++] = Op{static_cast<uint32_t*>(dst), static_cast<const uint32_t*>(src), bytes / 4};
+        if (bytes / 4 > words) words = bytes / 4;
+    }
+    void zero(void* dst, size_t bytes) { copy(dst, nullptr, bytes); }
+};
+__global__ void __launch_bounds__(256) control_batch_kernel(const __grid_constant__ ControlOps ops) {
+    for (int k = 0; k < ops.n; ++k) {
+        uint32_t* const dst = ops.op[k].dst;
+        const uint32_t* const src = ops.op[k].src;
+        const size_t n = ops.op[k].words;
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+            dst[i] = src ? src[i] : 0u;
+    }
 }
 static uint32_t control_grid(size_t n_words) {
     const size_t blocks = (n_words + 255) / 256;
@@ -238,13 +262,12 @@ static void control_copy(Context* c, void* dst, const void* src, size_t bytes, c
     CHK_CUDA(cudaGetLastError());
     c->launches++;
 }
-static void control_zero(Context* c, void* dst, size_t bytes, cudaStream_t s) {
-    if (bytes == 0) return;
-    control_fill_kernel<<<control_grid(bytes / 4), 256, 0, s>>>(static_cast<uint32_t*>(dst), bytes / 4);
+static void control_batch(Context* c, const ControlOps& ops, cudaStream_t s) {
+    if (!ops.n) return;
+    control_batch_kernel<<<control_grid(ops.words), 256, 0, s>>>(ops);
     CHK_CUDA(cudaGetLastError());
     c->launches++;
 }
-
 static void sync_stream(Context* c, cudaStream_t s) {
     if (!c->blocking_sync) {
         CHK_CUDA(cudaStreamSynchronize(s));
@@ -351,22 +374,6 @@ static std::string get_name(const uint8_t* p) {
     return std::string(reinterpret_cast<const char*>(p), n);
 }
 
-// Largest-first processing order of a batch plus a zeroed ticket counter for
-// the persistent encode / decode kernels.
-template <typename SizeFn>
-static void upload_order(Context* c, size_t W, SizeFn&& size_of) {
-    std::vector<uint32_t> order(W);
-    for (size_t i = 0; i < W; ++i) order[i] = (uint32_t)i;
-    std::stable_sort(order.begin(), order.end(),
-                     [&](uint32_t a, uint32_t b) { return size_of(a) > size_of(b); });
-    pin_ensure(c->h_order, W * 4);
-    std::memcpy(c->h_order.p, order.data(), W * 4);
-    dev_ensure(c, c->d_order, W * 4);
-    dev_ensure(c, c->d_ticket, 256);
-    control_copy(c, c->d_order.p, c->h_order.p, W * 4, c->stream);
-    control_zero(c, c->d_ticket.p, 256, c->stream);
-}
-
 // blocking: a host thread that waits for the event sleeps instead of spinning on a core
 static void ensure_events(std::vector<cudaEvent_t>& v, size_t n, bool timing, bool blocking = false) {
     while (v.size() < n) {
@@ -379,8 +386,9 @@ static void ensure_events(std::vector<cudaEvent_t>& v, size_t n, bool timing, bo
 
 // Grid of a persistent team kernel: as many teams as fit on the device at once.
 static uint32_t persistent_grid(Context* c, const void* kernel, size_t smem, size_t W, int cap_per_sm = 0) {
-    int per_sm = 0;
-    CHK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)kTeam, smem));
+    int& fit = c->resident_teams[kernel];
+    if (!fit) CHK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, (int)kTeam, smem));
+    int per_sm = fit;
     if (cap_per_sm > 0 && per_sm > cap_per_sm) per_sm = cap_per_sm;
     if (per_sm < 1) per_sm = 1;
     const size_t cap = (size_t)per_sm * (size_t)(c->sm_count > 0 ? c->sm_count : 1);
@@ -396,6 +404,9 @@ static uint32_t persistent_grid(Context* c, const void* kernel, size_t smem, siz
 //                  chains, lane and tensor offsets, headers and the gather into the data-section
 //                  layout, tensor by tensor inside the teams.  Its scratch is one slot per
 //                  resident team; a workspace bound simply means fewer teams.
+// When every tensor's lane regions fit the scratch that the resident teams would take ("direct"), the last step is
+// three launches instead -- lanes, offsets, gather (see rans_lanes_kernel) -- and the tables are not worth
+// overlapping.
 // Counting and encoding contend for the same units of an SM (shared-memory atomics against table
 // lookups): run side by side they only take turns, so they run one after the other, while the
 // memory-bound gather of finished tensors hides under the issue-bound chains of the others.
@@ -415,7 +426,7 @@ static void compress(Context* c, bool host_images) {
     pin_ensure(c->h_tiles, (W + 1) * 4);
     uint32_t* tile_start = static_cast<uint32_t*>(c->h_tiles.p);
     tile_start[0] = 0;
-    unsigned long long sidecar_total = 0, bytes_total = 0, slot_bytes = 0;
+    unsigned long long sidecar_total = 0, bytes_total = 0, slot_bytes = 0, regions_total = 0;
     uint32_t max_stride = 0;
     size_t n_sidecars = 0;
     bool any_member = false, any_int = false;
@@ -429,7 +440,6 @@ static void compress(Context* c, bool host_images) {
         d.spe = w.spe;
         d.table_idx = (uint32_t)w.table;
         d.sidecar_off = sidecar_total;
-        d.scratch_off = 0;  // lanes go to the slot of whichever team encodes the tensor
         const unsigned long long c_max = (w.bytes + 255) / 256;
         d.chunk_stride = (uint32_t)((2 * c_max + 31) & ~31ull);
         d.flags = w.owns ? kFlagNeedHist : 0u;
@@ -439,6 +449,8 @@ static void compress(Context* c, bool host_images) {
         // value-lane regions, plus one shared region for the lanes that only see zeroed bytes
         const unsigned long long need = (w.spe * 2 == w.es ? 129ull : 256ull) * d.chunk_stride;
         if (need > slot_bytes) slot_bytes = need;
+        d.scratch_off = regions_total;  // of its own (direct); the fused kernel's teams have a slot each and do not look
+        regions_total += need;
         if (d.chunk_stride > max_stride) max_stride = d.chunk_stride;
         bytes_total += w.bytes;
         n_sidecars += w.spe > 0;
@@ -466,27 +478,34 @@ static void compress(Context* c, bool host_images) {
         return;
     }
 
-    // ---- the encode grid and its scratch: one slot (the largest tensor's lane regions) per team
+    // ---- the encode grid and its scratch: one slot (the largest tensor's lane regions) per team, or a tensor's own
+    // regions for every tensor where that takes no more memory
     slot_bytes = (slot_bytes + 255) & ~255ull;
     auto kernel = any_int ? rans_encode_fused_kernel<true> : rans_encode_fused_kernel<false>;
+    auto lanes_kernel = any_int ? rans_lanes_kernel<true, false> : rans_lanes_kernel<false, false>;
     const size_t smem = any_int ? sizeof(EncSmem<4>) : sizeof(EncSmem<2>);
     uint32_t teams = persistent_grid(c, reinterpret_cast<const void*>(kernel), smem, W, c->encode_teams_per_sm);
-    if (c->workspace_bytes) {
+    const bool direct = c->workspace_bytes ? regions_total <= c->workspace_bytes : regions_total <= teams * slot_bytes;
+    if (direct) {
+        const size_t jobs = W + (W + kTeam - 1) / kTeam;  // the symbol-0 chains are teams too
+        teams = persistent_grid(c, reinterpret_cast<const void*>(lanes_kernel), smem, jobs, c->encode_teams_per_sm);
+    } else if (c->workspace_bytes) {
         const unsigned long long fit = c->workspace_bytes / slot_bytes;
         if (fit == 0)
             throw Error{CHK_ERR_CAPACITY, "workspace of " + std::to_string(c->workspace_bytes) + " bytes is smaller than the " +
                                               std::to_string(slot_bytes) + " bytes of encode scratch the largest tensor needs"};
         if (fit < teams) teams = (uint32_t)fit;
     }
+    const unsigned long long scratch_bytes = direct ? regions_total : (unsigned long long)teams * slot_bytes;
 
     // ---- pieces the batch is counted in (equal bytes; a small batch is one piece).  The tables of a piece are
     // built while the next piece is counted, so a piece must take about as long to count as the tables of the
     // one before take to build: a small last piece (1/16 of the bytes) exposed more table time, not less.
-    const size_t n_seg = W >= 512 && !c->precounted ? (size_t)c->segments : 1;
+    const size_t n_seg = !direct && W >= 512 && !c->precounted ? (size_t)c->segments : 1;
     std::vector<size_t> seg_end;
     {
         unsigned long long acc = 0;
-        for (size_t i = 0; i < W; ++i) {
+        for (size_t i = 0; i < W && n_seg > 1; ++i) {
             acc += c->descs[i].n_bytes;
             if (seg_end.size() + 1 < n_seg && acc * n_seg >= bytes_total * (seg_end.size() + 1)) seg_end.push_back(i + 1);
         }
@@ -499,17 +518,24 @@ static void compress(Context* c, bool host_images) {
     dev_ensure(c, c->d_tiles, (W + 1) * 4);
     dev_ensure(c, c->d_hist, W * 1024);
     dev_ensure(c, c->d_sidecar, sidecar_total + 64);
-    dev_ensure(c, c->d_scratch, (unsigned long long)teams * slot_bytes + 64);
+    dev_ensure(c, c->d_scratch, scratch_bytes + 64);
     // the batch's distinct symbol-0 chains (a handful: see zero_chain_kernel)
     const uint32_t z_slots = (uint32_t)(n_sidecars < 64 ? (n_sidecars ? n_sidecars : 1) : 64);
-    dev_ensure(c, c->d_zslots, z_slots * sizeof(ZeroSlot));
-    dev_ensure(c, c->d_zregions, (unsigned long long)z_slots * max_stride + 64);
-    dev_ensure(c, c->d_zslot_of, W * 4);
+    if (direct) {
+        dev_ensure(c, c->d_lane_src, W * kLanes * 8);
+        dev_ensure(c, c->d_lane_off, W * kLanes * 4);
+        dev_ensure(c, c->d_items, (W + 1) * 4);
+        pin_ensure(c->h_items, (W + 1) * 4);
+    } else {
+        dev_ensure(c, c->d_zslots, z_slots * sizeof(ZeroSlot));
+        dev_ensure(c, c->d_zregions, (unsigned long long)z_slots * max_stride + 64);
+        dev_ensure(c, c->d_zslot_of, W * 4);
+    }
     dev_ensure(c, c->d_hdrs, W * 4096);
     dev_ensure(c, c->d_ticket, 256);
     dev_ensure(c, c->d_order, W * 4);
     dev_ensure(c, c->d_psize, W * 8);
-    dev_ensure(c, c->d_payload, bytes_total + (unsigned long long)kPayloadAlign * W + 64);  // a heap: every range starts on a sector
+    dev_ensure(c, c->d_payload, bytes_total + (direct ? 0ull : (unsigned long long)kPayloadAlign * W) + 64);  // fused: a heap, every range starts on a sector
     dev_ensure(c, c->d_enc, T * 256 * sizeof(EncEntry));
     dev_ensure(c, c->d_freq, T * 256 * 4);
     dev_ensure(c, c->d_cum, T * 257 * 4);
@@ -540,21 +566,35 @@ static void compress(Context* c, bool host_images) {
         uint32_t* ord = static_cast<uint32_t*>(c->h_order.p);
         for (size_t i = 0; i < W; ++i) ord[i] = (uint32_t)i;
         std::stable_sort(ord, ord + W, [&](uint32_t x, uint32_t y) { return c->descs[x].n_bytes > c->descs[y].n_bytes; });
+        if (direct) {
+            uint32_t* items = static_cast<uint32_t*>(c->h_items.p);
+            items[0] = 0;
+            for (size_t i = 0; i < W; ++i) items[i + 1] = items[i] + kLanes * gather_pieces(c->descs[i].n_bytes);
+        }
     }
     ensure_events(c->ev_count, n_win, true);
     ensure_events(c->ev_tab, n_win, true);
 
     c->timing["prepare_ms"] = wall_ms(t_total);
     CHK_CUDA(cudaEventRecord(c->ev[0], s));
-    control_copy(c, c->d_descs.p, c->h_descs.p, W * sizeof(TensorDesc), s);
-    control_copy(c, c->d_tiles.p, c->h_tiles.p, (W + 1) * 4, s);
-    control_copy(c, c->d_jobs.p, c->h_jobs.p, T * sizeof(TableJob), s);
-    control_copy(c, c->d_order.p, c->h_order.p, W * 4, s);
-    if (!c->precounted) control_zero(c, c->d_hist.p, W * 1024, s);
-    control_zero(c, c->d_ticket.p, 256, s);  // word 0: ticket counter; words 2-3: the 64-bit heap cursor
-    control_zero(c, c->d_zslots.p, z_slots * sizeof(ZeroSlot), s);
+    {
+        ControlOps up;
+        up.copy(c->d_descs.p, c->h_descs.p, W * sizeof(TensorDesc));
+        up.copy(c->d_tiles.p, c->h_tiles.p, (W + 1) * 4);
+        up.copy(c->d_jobs.p, c->h_jobs.p, T * sizeof(TableJob));
+        up.copy(c->d_order.p, c->h_order.p, W * 4);
+        if (!c->precounted) up.zero(c->d_hist.p, W * 1024);
+        up.zero(c->d_ticket.p, 256);  // word 0: ticket counter; words 2-3: the 64-bit heap cursor; word 4: finished tensors
+        if (direct)
+            up.copy(c->d_items.p, c->h_items.p, (W + 1) * 4);
+        else
+            up.zero(c->d_zslots.p, z_slots * sizeof(ZeroSlot));
+        control_batch(c, up, s);
+    }
 
     const uint32_t sms = (uint32_t)(c->sm_count > 0 ? c->sm_count : 1);
+    uint8_t* const mt = host_images ? image_buffer(c, 1, kFileHeader + n_sidecars * kMantEntry + sidecar_total) : nullptr;
+    const size_t mt_data = kFileHeader + n_sidecars * kMantEntry;
     size_t tab_done = 0;
     for (size_t g = 0, a = 0; g < n_win; ++g) {
         const size_t b = seg_end[g], n = b - a;
@@ -573,11 +613,12 @@ static void compress(Context* c, bool host_images) {
         size_t tab_hi = tab_done;
         for (size_t i = a; i < b; ++i)
             if (c->work[i].owns) tab_hi = (size_t)c->work[i].table + 1;
-        CHK_CUDA(cudaStreamWaitEvent(c->side_stream, c->ev_count[g], 0));
+        const cudaStream_t ts = direct ? s : c->side_stream;
+        if (!direct) CHK_CUDA(cudaStreamWaitEvent(ts, c->ev_count[g], 0));
         if (tab_hi > tab_done) {
             const size_t t0 = tab_done, nt = tab_hi - tab_done;
             // a job's owner index counts from the start of the batch: whole-batch descriptor and histogram arrays
-            normalize_tables_kernel<<<(uint32_t)(nt < sms * 8u ? nt : sms * 8u), 256, 0, c->side_stream>>>(
+            normalize_tables_kernel<<<(uint32_t)(nt < sms * 8u ? nt : sms * 8u), 256, 0, ts>>>(
                 static_cast<const TableJob*>(c->d_jobs.p) + t0, static_cast<const TensorDesc*>(c->d_descs.p),
                 static_cast<const uint32_t*>(c->d_hist.p), static_cast<EncEntry*>(c->d_enc.p) + t0 * 256,
                 static_cast<uint32_t*>(c->d_freq.p) + t0 * 256, static_cast<uint32_t*>(c->d_cum.p) + t0 * 257,
@@ -586,47 +627,95 @@ static void compress(Context* c, bool host_images) {
             c->launches++;
             tab_done = tab_hi;
         }
-        // the symbol-0 chains this piece needs and the batch does not have yet
-        zero_chain_kernel<<<(uint32_t)n, 32, 0, c->side_stream>>>(
-            static_cast<const TensorDesc*>(c->d_descs.p) + a, static_cast<const EncEntry*>(c->d_enc.p),
-            static_cast<ZeroSlot*>(c->d_zslots.p), z_slots, static_cast<uint8_t*>(c->d_zregions.p), max_stride,
-            static_cast<int32_t*>(c->d_zslot_of.p) + a, (uint32_t)n);
-        CHK_CUDA(cudaGetLastError());
-        c->launches++;
-        CHK_CUDA(cudaEventRecord(c->ev_tab[g], c->side_stream));
+        if (!direct) {
+            // the symbol-0 chains this piece needs and the batch does not have yet
+            zero_chain_kernel<<<(uint32_t)n, 32, 0, ts>>>(
+                static_cast<const TensorDesc*>(c->d_descs.p) + a, static_cast<const EncEntry*>(c->d_enc.p),
+                static_cast<ZeroSlot*>(c->d_zslots.p), z_slots, static_cast<uint8_t*>(c->d_zregions.p), max_stride,
+                static_cast<int32_t*>(c->d_zslot_of.p) + a, (uint32_t)n);
+            CHK_CUDA(cudaGetLastError());
+            c->launches++;
+            CHK_CUDA(cudaEventRecord(c->ev_tab[g], ts));
+        }
         a = b;
     }
-    CHK_CUDA(cudaStreamWaitEvent(s, c->ev_tab[n_win - 1], 0));  // the table stream is in order: all tables are complete
+    if (!direct) CHK_CUDA(cudaStreamWaitEvent(s, c->ev_tab[n_win - 1], 0));  // the table stream is in order: all tables are complete
     CHK_CUDA(cudaEventRecord(c->ev[1], s));
     uint32_t* const ticket = static_cast<uint32_t*>(c->d_ticket.p);
-    FusedParams fp{};
-    fp.descs = static_cast<TensorDesc*>(c->d_descs.p);
-    fp.tables = static_cast<const EncEntry*>(c->d_enc.p);
-    fp.scratch = static_cast<uint8_t*>(c->d_scratch.p);
-    fp.slot_bytes = slot_bytes;
-    fp.zero_slots = static_cast<const ZeroSlot*>(c->d_zslots.p);
-    fp.zero_regions = static_cast<const uint8_t*>(c->d_zregions.p);
-    fp.zero_slot_of = static_cast<const int32_t*>(c->d_zslot_of.p);
-    fp.zero_region_stride = max_stride;
-    fp.n_tensors = (uint32_t)W;
-    fp.hdrs = static_cast<LaneHeader*>(c->d_hdrs.p);
-    fp.payload = static_cast<uint8_t*>(c->d_payload.p);
-    fp.payload_size = static_cast<unsigned long long*>(c->d_psize.p);
-    fp.heap_cursor = reinterpret_cast<unsigned long long*>(ticket + 2);
-    fp.order = static_cast<const uint32_t*>(c->d_order.p);
-    fp.ticket = ticket;
-    kernel<<<teams, kTeam, smem, s>>>(fp);
-    CHK_CUDA(cudaGetLastError());
-    c->launches++;
+    if (direct) {
+        LanesParams lp{};
+        lp.descs = static_cast<const TensorDesc*>(c->d_descs.p);
+        lp.tables = static_cast<const EncEntry*>(c->d_enc.p);
+        lp.scratch = static_cast<uint8_t*>(c->d_scratch.p);
+        lp.hdrs = static_cast<LaneHeader*>(c->d_hdrs.p);
+        lp.lane_src = static_cast<unsigned long long*>(c->d_lane_src.p);
+        lp.order = static_cast<const uint32_t*>(c->d_order.p);
+        lp.ticket = ticket;
+        lp.n_tensors = (uint32_t)W;
+        lanes_kernel<<<teams, kTeam, smem, s>>>(lp);
+        CHK_CUDA(cudaGetLastError());
+        OffsetsParams op{};
+        op.descs = static_cast<TensorDesc*>(c->d_descs.p);
+        op.hdrs = lp.hdrs;
+        op.lane_off = static_cast<uint32_t*>(c->d_lane_off.p);
+        op.payload_size = static_cast<unsigned long long*>(c->d_psize.p);
+        op.done = ticket + 4;
+        op.n_tensors = (uint32_t)W;
+        lane_offsets_kernel<<<(uint32_t)W, 256, 0, s>>>(op);
+        CHK_CUDA(cudaGetLastError());
+        const uint32_t items = static_cast<const uint32_t*>(c->h_items.p)[W], blocks = (items + 7) / 8;
+        gather_lanes_kernel<<<blocks < sms * 8u ? blocks : sms * 8u, 256, 0, s>>>(
+            lp.descs, static_cast<const uint32_t*>(c->d_items.p), lp.hdrs, lp.lane_src, op.lane_off, lp.scratch,
+            static_cast<uint8_t*>(c->d_payload.p), (uint32_t)W);
+        CHK_CUDA(cudaGetLastError());
+        c->launches += 3;
+    } else {
+        FusedParams fp{};
+        fp.descs = static_cast<TensorDesc*>(c->d_descs.p);
+        fp.tables = static_cast<const EncEntry*>(c->d_enc.p);
+        fp.scratch = static_cast<uint8_t*>(c->d_scratch.p);
+        fp.slot_bytes = slot_bytes;
+        fp.zero_slots = static_cast<const ZeroSlot*>(c->d_zslots.p);
+        fp.zero_regions = static_cast<const uint8_t*>(c->d_zregions.p);
+        fp.zero_slot_of = static_cast<const int32_t*>(c->d_zslot_of.p);
+        fp.zero_region_stride = max_stride;
+        fp.n_tensors = (uint32_t)W;
+        fp.hdrs = static_cast<LaneHeader*>(c->d_hdrs.p);
+        fp.payload = static_cast<uint8_t*>(c->d_payload.p);
+        fp.payload_size = static_cast<unsigned long long*>(c->d_psize.p);
+        fp.heap_cursor = reinterpret_cast<unsigned long long*>(ticket + 2);
+        fp.order = static_cast<const uint32_t*>(c->d_order.p);
+        fp.ticket = ticket;
+        kernel<<<teams, kTeam, smem, s>>>(fp);
+        CHK_CUDA(cudaGetLastError());
+        c->launches++;
+    }
     CHK_CUDA(cudaEventRecord(c->ev[2], s));
     c->timing["enqueue_ms"] = wall_ms(t_total);
+    // the low bytes are complete once everything is counted: they cross to the host while the lanes are encoded
+    struct SideWork {  // whatever ends this call, the copy is done before its buffers are used again
+        cudaStream_t s = nullptr;
+        ~SideWork() {
+            if (s) cudaStreamSynchronize(s);
+        }
+    } side_work;
+    if (host_images && sidecar_total) {
+        side_work.s = c->side_stream;
+        CHK_CUDA(cudaStreamWaitEvent(c->side_stream, c->ev_count[n_win - 1], 0));
+        CHK_CUDA(cudaMemcpyAsync(mt + mt_data, c->d_sidecar.p, sidecar_total, cudaMemcpyDeviceToHost, c->side_stream));
+        CHK_CUDA(cudaEventRecord(c->ev[7], c->side_stream));
+    }
 
-    control_copy(c, c->h_psize.p, c->d_psize.p, W * 8, s);
-    control_copy(c, c->h_descs.p, c->d_descs.p, W * sizeof(TensorDesc), s);
-    control_copy(c, c->h_sums.p, c->d_sums.p, T * 4, s);
-    if (host_images) control_copy(c, c->h_hdrs.p, c->d_hdrs.p, W * 4096, s);
-    if (want_tables) control_copy(c, c->h_freq.p, c->d_freq.p, T * 256 * 4, s);
-    if (host_images) control_copy(c, c->h_cum.p, c->d_cum.p, T * 257 * 4, s);
+    {
+        ControlOps down;
+        down.copy(c->h_psize.p, c->d_psize.p, W * 8);
+        if (!direct) down.copy(c->h_descs.p, c->d_descs.p, W * sizeof(TensorDesc));  // where in the heap each payload is
+        down.copy(c->h_sums.p, c->d_sums.p, T * 4);
+        if (host_images) down.copy(c->h_hdrs.p, c->d_hdrs.p, W * 4096);
+        if (want_tables) down.copy(c->h_freq.p, c->d_freq.p, T * 256 * 4);
+        if (host_images) down.copy(c->h_cum.p, c->d_cum.p, T * 257 * 4);
+        control_batch(c, down, s);
+    }
     sync_stream(c, s);
 
     c->timing["split_hist_ms"] = ms_between(c->ev[0], c->ev_count[n_win - 1]);
@@ -636,16 +725,23 @@ static void compress(Context* c, bool host_images) {
     c->timing["device_span_ms"] = ms_between(c->ev[0], c->ev[2]);
     c->timing["compress_device_ms"] = c->timing["device_span_ms"];
     c->timing["encode_teams"] = (double)teams;
-    c->timing["workspace_mb"] = (double)((unsigned long long)teams * slot_bytes) / 1048576.0;
+    c->timing["workspace_mb"] = (double)scratch_bytes / 1048576.0;
     c->timing["to_sync_ms"] = wall_ms(t_total);
 
-    // descriptors come back with each tensor's place in the payload heap and its raw flag; the file wants
-    // the payloads in index order, so the offsets written there are the running sum of the sizes
-    std::memcpy(c->descs.data(), c->h_descs.p, W * sizeof(TensorDesc));
+    // The file wants the payloads in index order: offsets there are the running sum of the sizes.  The direct path has
+    // laid them out like that; after the fused kernel the descriptors come back with each tensor's place in the heap.
     const unsigned long long* psize = static_cast<const unsigned long long*>(c->h_psize.p);
     unsigned long long* poff = static_cast<unsigned long long*>(c->h_poff.p);
     poff[0] = 0;
     for (size_t i = 0; i < W; ++i) poff[i + 1] = poff[i] + psize[i];
+    if (direct) {
+        for (size_t i = 0; i < W; ++i) {
+            c->descs[i].payload_off = poff[i];
+            if (psize[i] == c->descs[i].n_bytes) c->descs[i].flags |= kFlagRaw;  // a coded payload is smaller than its tensor
+        }
+    } else {
+        std::memcpy(c->descs.data(), c->h_descs.p, W * sizeof(TensorDesc));
+    }
     const unsigned long long payload_total = poff[W];
     const uint32_t* sums = static_cast<const uint32_t*>(c->h_sums.p);
     c->table_sums.assign(sums, sums + T);
@@ -678,7 +774,8 @@ static void compress(Context* c, bool host_images) {
         uint8_t* st = image_buffer(c, 0, c->summary.states_bytes);
         const size_t st_data = kFileHeader + W * kStatesEntry;
         // heap order -> file order on the device, then the data section in one copy
-        if (payload_total) {
+        const void* section = c->d_payload.p;
+        if (payload_total && !direct) {
             dev_ensure(c, c->d_poff, (W + 1) * 8);
             dev_ensure(c, c->d_fileorder, payload_total + 64);
             control_copy(c, c->d_poff.p, c->h_poff.p, (W + 1) * 8, s);
@@ -689,13 +786,10 @@ static void compress(Context* c, bool host_images) {
                 static_cast<uint8_t*>(c->d_fileorder.p), (uint32_t)W);
             CHK_CUDA(cudaGetLastError());
             c->launches++;
-            CHK_CUDA(cudaMemcpyAsync(st + st_data, c->d_fileorder.p, payload_total, cudaMemcpyDeviceToHost, s));
+            section = c->d_fileorder.p;
         }
-        // mantissa image (write_rank_mantissa_file, :839-887)
-        uint8_t* mt = image_buffer(c, 1, c->summary.mantissa_bytes);
-        const size_t mt_data = kFileHeader + n_sidecars * kMantEntry;
-        if (sidecar_total)
-            CHK_CUDA(cudaMemcpyAsync(mt + mt_data, c->d_sidecar.p, sidecar_total, cudaMemcpyDeviceToHost, s));
+        if (payload_total) CHK_CUDA(cudaMemcpyAsync(st + st_data, section, payload_total, cudaMemcpyDeviceToHost, s));
+        if (sidecar_total) CHK_CUDA(cudaStreamWaitEvent(s, c->ev[7], 0));  // the mantissa image (write_rank_mantissa_file, :839-887)
         // tables image (write_rank_tables_file, :903-931)
         uint8_t* dc = image_buffer(c, 2, c->summary.dict_bytes);
 
@@ -754,6 +848,7 @@ static void compress(Context* c, bool host_images) {
         }
         CHK_CUDA(cudaEventRecord(c->ev[6], s));
         sync_stream(c, s);
+        side_work.s = nullptr;
         c->timing["d2h_ms"] = ms_between(c->ev[5], c->ev[6]);
         c->have_images = true;
     }
@@ -798,34 +893,40 @@ static void compress_and_save(Context* c, const std::string& dir) {
 }
 
 // ------------------------------------------------------------------ restore
+// Decodes the W tensors described in h_descs (uploaded here together with their order).
 static void run_decode(Context* c, size_t W, const uint8_t* d_payload, const uint8_t* d_sidecar,
                        const uint32_t* d_freq, const uint32_t* d_cum, const LaneHeader* d_hdrs,
                        const std::vector<size_t>& tensor_of) {
     cudaStream_t s = c->stream;
-    dev_ensure(c, c->d_status, W * 4 + 256);
+    // One status word per tensor in pinned host memory: the kernels write it only when a stream check fails, so it costs
+    // neither a clearing launch nor a copy back.
     pin_ensure(c->h_status, W * 4 + 256);
-    control_zero(c, c->d_status.p, W * 4, s);
+    std::memset(c->h_status.p, 0, W * 4);
     // Two launches at most.  With option "decode_zero_skip", floating-point tensors whose table gives symbol 0
     // half of the slots (all of them, as a rule) go to the kernel with the short table, of which more teams fit an
-    // SM; integer tensors -- four chains per thread, larger rings -- and whatever does not qualify go to the
+    // SM; integer tensors -- two chains per thread, larger rings -- and whatever does not qualify go to the
     // full-table kernel.  Off by default: on a B200 the two extra instructions per symbol cost more than the
-    // added teams bring (9.8 ms against 9.6 ms for the 14 GB benchmark shard).
+    // added teams bring.
     const TensorDesc* hd = static_cast<const TensorDesc*>(c->h_descs.p);
-    std::vector<uint32_t> order(W);
+    pin_ensure(c->h_order, W * 4);
+    uint32_t* const order = static_cast<uint32_t*>(c->h_order.p);
     for (size_t i = 0; i < W; ++i) order[i] = (uint32_t)i;
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return hd[a].n_bytes > hd[b].n_bytes; });
-    auto short_table = [&](uint32_t i) {
-        return c->decode_zero_skip && hd[i].spe * 2 == hd[i].es && (hd[i].flags & kFlagZeroSkip) && !(hd[i].flags & kFlagRaw);
-    };
-    const size_t n_short = (size_t)(std::stable_partition(order.begin(), order.end(), short_table) - order.begin());
+    std::stable_sort(order, order + W, [&](uint32_t a, uint32_t b) { return hd[a].n_bytes > hd[b].n_bytes; });
+    size_t n_short = 0;
+    if (c->decode_zero_skip)
+        n_short = (size_t)(std::stable_partition(order, order + W, [&](uint32_t i) {
+                               return hd[i].spe * 2 == hd[i].es && (hd[i].flags & kFlagZeroSkip) && !(hd[i].flags & kFlagRaw);
+                           }) - order);
     bool any_int = false;
     for (size_t k = n_short; k < W && !any_int; ++k) any_int = hd[order[k]].spe * 2 != hd[order[k]].es;
-    pin_ensure(c->h_order, W * 4);
-    std::memcpy(c->h_order.p, order.data(), W * 4);
+    dev_ensure(c, c->d_descs, W * sizeof(TensorDesc));
     dev_ensure(c, c->d_order, W * 4);
     dev_ensure(c, c->d_ticket, 256);
-    control_copy(c, c->d_order.p, c->h_order.p, W * 4, s);
-    control_zero(c, c->d_ticket.p, 256, s);
+    ControlOps up;
+    up.copy(c->d_descs.p, c->h_descs.p, W * sizeof(TensorDesc));
+    up.copy(c->d_order.p, order, W * 4);
+    up.zero(c->d_ticket.p, 256);
+    control_batch(c, up, s);
     CHK_CUDA(cudaEventRecord(c->ev[1], s));
     auto launch = [&](auto kernel, uint32_t smem, size_t first, size_t n, uint32_t ticket_word) {
         if (!n) return;
@@ -833,21 +934,21 @@ static void run_decode(Context* c, size_t W, const uint8_t* d_payload, const uin
         kernel<<<grid, kTeam, smem, s>>>(static_cast<const TensorDesc*>(c->d_descs.p), d_freq, d_cum, d_hdrs, d_payload,
                                          d_sidecar, static_cast<const uint32_t*>(c->d_order.p) + first,
                                          static_cast<uint32_t*>(c->d_ticket.p) + ticket_word, (uint32_t)n,
-                                         c->verify_zero_lanes ? 1u : 0u, static_cast<uint32_t*>(c->d_status.p));
+                                         c->verify_zero_lanes ? 1u : 0u, static_cast<uint32_t*>(c->h_status.p));
         CHK_CUDA(cudaGetLastError());
         c->launches++;
     };
     launch(rans_decode_kernel<false, true>, kDecSmemBytes[0][1], 0, n_short, 0);
+    // up to two teams an SM a scheduler has two warps at most, and a chain's latency is what counts (see dec_step)
+    const size_t n = W - n_short;
+    const bool few = n <= 2 * (size_t)(c->sm_count > 0 ? c->sm_count : 1);
     if (any_int)
-        launch(rans_decode_kernel<true, false>, kDecSmemBytes[1][0], n_short, W - n_short, 8);
+        launch(few ? rans_decode_kernel<true, false, true> : rans_decode_kernel<true, false, false>, kDecSmemBytes[1][0], n_short, n, 8);
     else
-        launch(rans_decode_kernel<false, false>, kDecSmemBytes[0][0], n_short, W - n_short, 8);
+        launch(few ? rans_decode_kernel<false, false, true> : rans_decode_kernel<false, false, false>, kDecSmemBytes[0][0], n_short, n, 8);
     CHK_CUDA(cudaEventRecord(c->ev[2], s));
-    control_copy(c, c->h_status.p, c->d_status.p, W * 4, s);
-    CHK_CUDA(cudaEventRecord(c->ev[4], s));
     sync_stream(c, s);
     c->timing["decode_ms"] = ms_between(c->ev[1], c->ev[2]);
-    c->timing["decode_tail_ms"] = ms_between(c->ev[2], c->ev[4]);
     const uint32_t* st = static_cast<const uint32_t*>(c->h_status.p);
     for (size_t i = 0; i < W; ++i)
         if (st[i])
@@ -898,8 +999,6 @@ static void decompress_resident(Context* c, void* const* dst) {
     if (!all) throw Error{CHK_ERR_INVALID, "chk_decompress_resident: partial restore is not supported; pass all targets"};
     pin_ensure(c->h_descs, W * sizeof(TensorDesc));
     std::memcpy(c->h_descs.p, run.data(), W * sizeof(TensorDesc));
-    dev_ensure(c, c->d_descs, W * sizeof(TensorDesc));
-    control_copy(c, c->d_descs.p, c->h_descs.p, W * sizeof(TensorDesc), c->stream);
     run_decode(c, W, static_cast<const uint8_t*>(c->d_payload.p), static_cast<const uint8_t*>(c->d_sidecar.p),
                static_cast<const uint32_t*>(c->d_freq.p), static_cast<const uint32_t*>(c->d_cum.p),
                static_cast<const LaneHeader*>(c->d_hdrs.p), tensor_of);
@@ -1001,7 +1100,6 @@ static void decompress_images(Context* c, const uint8_t* st, size_t st_n, const 
     if (W == 0) return;
 
     cudaStream_t s = c->stream;
-    dev_ensure(c, c->d_descs, W * sizeof(TensorDesc));
     dev_ensure(c, c->d_payload, payload_total + 64);
     dev_ensure(c, c->d_sidecar, sidecar_total + 64);
     dev_ensure(c, c->d_hdrs, W * 4096);
@@ -1012,7 +1110,6 @@ static void decompress_images(Context* c, const uint8_t* st, size_t st_n, const 
 
     c->timing["parse_ms"] = wall_ms(t_total);
     CHK_CUDA(cudaEventRecord(c->ev[0], s));
-    control_copy(c, c->d_descs.p, c->h_descs.p, W * sizeof(TensorDesc), s);
     // index data first, so it does not queue behind this call's own bulk copies
     // lane headers: one strided copy per run of consecutive entries
     for (size_t k = 0; k < W;) {
@@ -1383,7 +1480,7 @@ static void release_device_buffers(chk_context* c) {
     if (c->side_stream) cudaStreamSynchronize(c->side_stream);
     DevBuf* bufs[] = {&c->d_descs, &c->d_tiles, &c->d_hist, &c->d_sidecar, &c->d_scratch, &c->d_hdrs,
                       &c->d_order, &c->d_ticket, &c->d_psize, &c->d_zslots, &c->d_zregions, &c->d_zslot_of, &c->d_jobs, &c->d_sums, &c->d_payload, &c->d_enc,
-                      &c->d_freq, &c->d_cum, &c->d_status, &c->d_stats_desc, &c->d_stats_out, &c->d_stats_part, &c->d_stats_mid, &c->d_poff, &c->d_fileorder, &c->d_hll32, &c->d_hll8, &c->d_symkeys, &c->d_symcounts};
+                      &c->d_freq, &c->d_cum, &c->d_stats_desc, &c->d_stats_out, &c->d_stats_part, &c->d_stats_mid, &c->d_poff, &c->d_fileorder, &c->d_lane_src, &c->d_lane_off, &c->d_items, &c->d_hll32, &c->d_hll8, &c->d_symkeys, &c->d_symcounts};
     for (DevBuf* b : bufs) {
         if (b->p) cudaFreeAsync(b->p, c->stream);
         b->p = nullptr;
@@ -1409,7 +1506,7 @@ int chk_context_destroy(chk_context* c) {
     cudaSetDevice(c->device);
     v3_destroy(c);
     release_device_buffers(c);
-    PinBuf* pins[] = {&c->h_hdrs, &c->h_poff, &c->h_psize, &c->h_descs, &c->h_status, &c->h_jobs, &c->h_sums, &c->h_freq, &c->h_cum, &c->h_stats, &c->h_order, &c->h_tiles,
+    PinBuf* pins[] = {&c->h_hdrs, &c->h_poff, &c->h_psize, &c->h_descs, &c->h_status, &c->h_jobs, &c->h_sums, &c->h_freq, &c->h_cum, &c->h_stats, &c->h_order, &c->h_tiles, &c->h_items,
                       &c->img[0], &c->img[1], &c->img[2]};
     for (PinBuf* b : pins)
         if (b->p) cudaFreeHost(b->p);

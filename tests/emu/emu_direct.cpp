@@ -1,0 +1,78 @@
+// emu_direct.cpp -- the kernels of the one-batch ("direct") encode path on the CPU block emulator: lanes with the
+// symbol-0 chains as teams of the same launch, offsets with the tensor scan in the last block, gather in pieces.
+// Test-only; built by tests/test_direct_encode.py.
+#include "cuda_emu.hpp"
+//
+#include "kernels.cuh"
+#include "tables.hpp"
+
+#include <vector>
+
+using namespace chk;
+
+extern "C" {
+
+// payload_off_out: n + 1 entries; hdrs_out: n * 1024 words; raw_out: n bytes.
+void emu_encode_direct(size_t n, const uint8_t* const* srcs, const uint64_t* n_bytes, const uint32_t* es, const uint32_t* spe,
+                       const uint32_t* nf, const uint32_t* cf, uint8_t* payload_out, uint64_t* payload_off_out,
+                       uint32_t* hdrs_out, uint8_t* raw_out, uint32_t grid, uint32_t ints, uint32_t escape) {
+    std::vector<TensorDesc> descs(n);
+    std::vector<uint32_t> items(n + 1, 0), order(n);
+    unsigned long long scratch_total = 0;
+    for (size_t i = 0; i < n; ++i) {
+        TensorDesc& d = descs[i];
+        std::memset(&d, 0, sizeof(d));
+        d.src = srcs[i];
+        d.n_bytes = n_bytes[i];
+        d.es = es[i];
+        d.spe = spe[i];
+        d.table_idx = (uint32_t)i;
+        d.chunk_stride = (uint32_t)((2 * ((d.n_bytes + 255) / 256) + 31) & ~31ull);
+        d.scratch_off = scratch_total;
+        scratch_total += (d.spe * 2 == d.es ? 129ull : 256ull) * d.chunk_stride;
+        items[i + 1] = items[i] + kLanes * gather_pieces(d.n_bytes);
+        order[i] = (uint32_t)(n - 1 - i);
+    }
+    std::vector<EncEntry> enc(n * 256);
+    for (size_t t = 0; t < n; ++t) {
+        FreqTable ft;
+        std::memcpy(ft.norm_freq, nf + t * 256, 1024);
+        std::memcpy(ft.cum_freq, cf + t * 257, 1028);
+        build_enc_entries(ft, &enc[t * 256]);
+    }
+    std::vector<uint8_t> scratch(scratch_total + 64, 0xAA);
+    uint8_t* scr = (uint8_t*)(((uintptr_t)scratch.data() + 31) & ~(uintptr_t)31);
+    std::vector<LaneHeader> hdrs(n * 256);
+    std::vector<unsigned long long> lsrc(n * 256), psize(n);
+    std::vector<uint32_t> loff(n * 256);
+    uint32_t ticket = 0, done = 0;
+    LanesParams lp{descs.data(), enc.data(), scr, hdrs.data(), lsrc.data(), order.data(), &ticket, (uint32_t)n};
+    if (ints && escape)
+        emu::launch(grid, kTeam, sizeof(EncSmem<4>), [&] { rans_lanes_kernel<true, true>(lp); });
+    else if (ints)
+        emu::launch(grid, kTeam, sizeof(EncSmem<4>), [&] { rans_lanes_kernel<true, false>(lp); });
+    else
+        emu::launch(grid, kTeam, sizeof(EncSmem<2>), [&] { rans_lanes_kernel<false, false>(lp); });
+    OffsetsParams op{descs.data(), hdrs.data(), loff.data(), psize.data(), &done, (uint32_t)n};
+    emu::launch((unsigned)n, 256, 0, [&] { lane_offsets_kernel(op); });
+    emu::launch(grid, 256, 0, [&] {
+        gather_lanes_kernel(descs.data(), items.data(), hdrs.data(), lsrc.data(), loff.data(), scr, payload_out, (uint32_t)n);
+    });
+    payload_off_out[0] = 0;
+    for (size_t i = 0; i < n; ++i) {
+        payload_off_out[i] = descs[i].payload_off;
+        payload_off_out[i + 1] = descs[i].payload_off + psize[i];
+        raw_out[i] = (descs[i].flags & kFlagRaw) ? 1 : 0;
+    }
+    std::memcpy(hdrs_out, hdrs.data(), n * 4096);
+}
+
+// The order block_sort_order gives n keys (symbols 0 .. n-1 in input order): position of every symbol.
+void emu_block_sort(size_t n, const double* frac, int32_t* place_out) {
+    static NormSmem sm;
+    for (size_t i = 0; i < n; ++i) sm.keys[i] = FracKey{frac[i], (int32_t)i, 0};
+    emu::launch(1, 256, 0, [&] { block_sort_order(sm, (uint32_t)n); });
+    for (size_t i = 0; i < n; ++i) place_out[i] = sm.place[i];
+}
+
+}  // extern "C"

@@ -1,0 +1,149 @@
+"""The one-batch encode path (rans_lanes_kernel, lane_offsets_kernel, gather_lanes_kernel), bit-exact against the
+oracle: on the CPU block emulator, and on the GPU through file images.  Sizes sit at the edges the kernels have: rows
+of 256 bytes, groups of 16 rows (4096 bytes), a partial row, lanes longer than one gather piece, more tensors than a
+team has threads (a second group of symbol-0 chains)."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from emu_lib import CSRC, EMU_DIR, aligned
+from oracle_lib import ELEM_SIZE, SIDECAR_PER_ELEM, synth
+
+EDGES = [1, 255, 256, 257, 4095, 4096, 4097, 8192, 3 * 4096 + 256, 3 * 4096 + 257, 16 * 4096]  # bytes
+u8p, u32p, u64p = C.POINTER(C.c_uint8), C.POINTER(C.c_uint32), C.POINTER(C.c_uint64)
+
+
+@pytest.fixture(scope="module")
+def direct_lib():
+    so = os.path.join(EMU_DIR, "libemu_direct.so")
+    srcs = [os.path.join(EMU_DIR, f) for f in ("emu_direct.cpp", "cuda_emu.hpp")] + \
+           [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    if not os.path.exists(so) or any(os.path.getmtime(so) < os.path.getmtime(s) for s in srcs):
+        subprocess.check_call(["g++", "-std=c++17", "-O1", "-I", CSRC, "-I", EMU_DIR, "-shared", "-fPIC", "-w", srcs[0], "-o", so])
+    return C.CDLL(so)
+
+
+@pytest.fixture(scope="module")
+def direct(direct_lib):
+    lib = direct_lib
+
+    def encode(tensors, es, spe, nf, cf, grid, ints, escape=False):
+        n = len(tensors)
+        ptrs = (C.c_void_p * n)(*[t.ctypes.data for t in tensors])
+        nb = np.array([t.size for t in tensors], np.uint64)
+        e, s = np.array(es, np.uint32), np.array(spe, np.uint32)
+        nf, cf = np.ascontiguousarray(nf, np.uint32), np.ascontiguousarray(cf, np.uint32)
+        payload, off = aligned(int(nb.sum()) + 64, fill=0xCC), np.zeros(n + 1, np.uint64)
+        hdrs, raw = np.zeros((n, 256, 4), np.uint32), np.zeros(n, np.uint8)
+        p = lambda a, t: a.ctypes.data_as(t)  # noqa: E731
+        lib.emu_encode_direct(C.c_size_t(n), ptrs, p(nb, u64p), p(e, u32p), p(s, u32p), p(nf, u32p), p(cf, u32p),
+                              p(payload, u8p), p(off, u64p), p(hdrs, u32p), p(raw, u8p), C.c_uint32(grid),
+                              C.c_uint32(int(ints)), C.c_uint32(int(escape)))
+        return payload, off, hdrs, raw
+
+    return encode
+
+
+def batch(kinds, misalign):
+    out = []
+    for i, (kind, n) in enumerate(kinds):
+        raw, dt = synth(kind, n, 500 + i)
+        m = misalign[i % len(misalign)] * ELEM_SIZE[dt]
+        a = aligned(raw.size + 64)[m:m + raw.size]
+        a[:] = raw
+        out.append((a, dt))
+    return out
+
+
+def tables(oracle, tensors):
+    masked, tabs = [], []
+    for a, dt in tensors:
+        masked.append(oracle.split(a, dt)[0] if SIDECAR_PER_ELEM[dt] else a.copy())
+        tabs.append(oracle.normalize(oracle.byte_histogram(masked[-1]), False))
+    return masked, tabs
+
+
+@pytest.mark.parametrize("kind", ["f32_master", "bf16_weight", "f32_exp_avg_sq_lognormal", "i8", "mixed"])
+@pytest.mark.parametrize("misalign", [[0], [1, 0, 3]])
+def test_lanes_offsets_gather(direct, oracle, kind, misalign):
+    if kind == "mixed":  # 130 tensors: two groups of symbol-0 chains
+        kinds = [(k, 1 + (37 * i) % 400) for i in range(44) for k in ("f32_master", "bf16_weight", "i8")]
+    else:
+        es = ELEM_SIZE[synth(kind, 1, 0)[1]]
+        kinds = [(kind, max(1, b // es)) for b in EDGES]
+        if kind == "f32_master":
+            kinds.append((kind, 300_000))  # 4688 rows: lanes of more than one gather piece under a borrowed-table worst case
+    tensors = batch(kinds, misalign)
+    masked, tabs = tables(oracle, tensors)
+    es, spe = [ELEM_SIZE[d] for _, d in tensors], [SIDECAR_PER_ELEM[d] for _, d in tensors]
+    ints = any(2 * s != e for e, s in zip(es, spe))
+    payload, off, hdrs, raw = direct([a for a, _ in tensors], es, spe, np.stack([t[0] for t in tabs]),
+                                     np.stack([t[1] for t in tabs]), 5, ints)
+    for i, (m, t) in enumerate(zip(masked, tabs)):
+        p, h, r = oracle.compress_tensor(m, *t[:3])
+        assert bool(raw[i]) == r, kinds[i]
+        assert np.array_equal(payload[int(off[i]):int(off[i + 1])], p), kinds[i]
+        assert np.array_equal(hdrs[i], h), kinds[i]
+    assert np.all(payload[int(off[-1]):] == 0xCC)  # nothing is written behind the data section
+
+
+def test_long_lanes_and_escapes(direct, oracle):
+    """A lane of several gather pieces (12-bit codes for every value byte), and symbols a borrowed table lacks."""
+    tensors = batch([("f32_uniform_bits", 1_100_000), ("f32_master", 5000)], [0])
+    masked, _ = tables(oracle, tensors)
+    hist_skew = np.ones(256, np.uint32)
+    hist_skew[0] = 10 ** 6
+    hist_few = np.zeros(256, np.uint32)
+    hist_few[:4] = [100, 50, 20, 3]
+    tabs = [oracle.normalize(hist_skew, False), oracle.normalize(hist_few, False)]
+    nf, cf = np.stack([t[0] for t in tabs]), np.stack([t[1] for t in tabs])
+    payload, off, hdrs, raw = direct([a for a, _ in tensors], [4, 4], [2, 2], nf, cf, 3, True, escape=True)
+    for i in range(2):
+        p, h, r = oracle.compress_tensor(masked[i], *tabs[i][:3])
+        assert bool(raw[i]) == r and np.array_equal(payload[int(off[i]):int(off[i + 1])], p), i
+        assert np.array_equal(hdrs[i], h), i
+    assert hdrs[0][:, 1].max() > 8192
+
+
+@pytest.mark.parametrize("n", [2, 16, 17, 33, 64, 255, 256])
+def test_block_sort_leaves_the_order_of_std_sort(direct_lib, emu, n):
+    """Ties of every density, sorted and reversed input, and the input on which the library falls back to its heap sort."""
+    f64p, i32p = C.POINTER(C.c_double), C.POINTER(C.c_int32)
+    rng = np.random.default_rng(n)
+    inputs = [rng.integers(0, d, n) / d for d in (1, 2, 5, 40, 10 ** 6) for _ in range(6)]
+    inputs += [np.arange(n, dtype=float), np.arange(n, 0, -1, dtype=float), np.repeat(np.arange((n + 2) // 3), 3)[:n].astype(float)]
+    killer = np.zeros(n, np.float64)
+    emu.lib.emu_sort_killer(C.c_size_t(n), killer.ctypes.data_as(f64p))
+    inputs += [np.floor(killer / c) for c in (1, 3, 7)]
+    for frac in inputs:
+        frac = np.ascontiguousarray(frac, np.float64)
+        place, order = np.zeros(n, np.int32), np.zeros(n, np.int32)
+        direct_lib.emu_block_sort(C.c_size_t(n), frac.ctypes.data_as(f64p), place.ctypes.data_as(i32p))
+        emu.lib.emu_std_sort(C.c_size_t(n), frac.ctypes.data_as(f64p), order.ctypes.data_as(i32p))
+        assert np.array_equal(np.argsort(place), order), frac
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("workspace", [0, 1 << 20])
+def test_files_on_the_device(oracle, tmp_path, workspace):
+    """Direct (no bound: every tensor has scratch of its own) and fused (bounded: teams share slots) give the oracle's files."""
+    torch = pytest.importorskip("torch")
+    import checkers_b200 as chk
+    kinds = [(k, max(1, b // e)) for b in EDGES for k, e in (("f32_master", 4), ("bf16_weight", 2), ("i8", 1))]
+    kinds.append(("f32_master", 300_000))
+    host = [synth(k, n, 60 + i) for i, (k, n) in enumerate(kinds)]
+    names = [f"t{i}" for i in range(len(host))]
+    dev = [torch.from_numpy(np.concatenate([raw, np.zeros(16, np.uint8)])).cuda() for raw, _ in host]
+    torch.cuda.synchronize()
+    need = max((129 if dt != 3 else 256) * (2 * (-(-raw.size // 256)) + 31) for raw, dt in host)
+    ctx = chk.Context(device=0, workspace_bytes=max(workspace, need) if workspace else 0)
+    for nm, d, (raw, dt) in zip(names, dev, host):
+        ctx.register_pointer(nm, d.data_ptr(), raw.size // ELEM_SIZE[dt], dt)
+    ctx.compress_and_save(str(tmp_path / "gpu"))
+    oracle.compress_and_save(names, [r for r, _ in host], [d for _, d in host], str(tmp_path / "cpu"))
+    for rel in ("rank_0_states.ansc", "mantissa/rank_0_mantissa.mant", "tables/rank_0_tables.dict"):
+        assert (tmp_path / "gpu" / rel).read_bytes() == (tmp_path / "cpu" / rel).read_bytes(), rel
+    ctx.close()
