@@ -893,6 +893,31 @@ static void compress_and_save(Context* c, const std::string& dir) {
 }
 
 // ------------------------------------------------------------------ restore
+// Whether a batch of `units` (128 chains each, `rows` rows in all) goes to rans_decode_split_kernel.  Its steps are
+// cheaper, its start is dearer (256 or 384 threads and a slot table per unit): it wins whenever the units fit the device
+// at once, and past that from about 200 rows a unit on (4096 tensors of 128 rows: 0.122 against 0.124 ms, of 64 rows
+// 0.30 against 0.26).  Integer tensors are two units with a table each where the other kernel builds one: for those it
+// wins only as long as there is room for them (1024 tensors of 128 KiB: 0.22 against 0.17 ms).
+static bool prefer_split(size_t units, size_t int_units, uint64_t rows, size_t sms) {
+    if (2 * int_units > units) return units <= 2 * sms;
+    return units <= 4 * sms || rows >= 256 * (uint64_t)units;
+}
+template <int kKind>
+static void launch_split(Context* c, const SplitParams& fp, cudaStream_t s) {
+    auto kernel = rans_decode_split_kernel<kKind>;
+    constexpr uint32_t threads = SplitSmem<kKind>::kChains + kSplitHelpers, smem = (uint32_t)sizeof(SplitSmem<kKind>);
+    int& fit = c->resident_teams[reinterpret_cast<const void*>(kernel)];
+    if (!fit) {
+        CHK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CHK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, (int)threads, smem));
+        if (fit < 1) fit = 1;
+    }
+    const size_t cap = (size_t)fit * (size_t)(c->sm_count > 0 ? c->sm_count : 1);
+    kernel<<<(uint32_t)(fp.n_units < cap ? fp.n_units : cap), threads, smem, s>>>(fp);
+    CHK_CUDA(cudaGetLastError());
+    c->launches++;
+}
+
 // Decodes the W tensors described in h_descs (uploaded here together with their order).
 static void run_decode(Context* c, size_t W, const uint8_t* d_payload, const uint8_t* d_sidecar,
                        const uint32_t* d_freq, const uint32_t* d_cum, const LaneHeader* d_hdrs,
@@ -908,7 +933,7 @@ static void run_decode(Context* c, size_t W, const uint8_t* d_payload, const uin
     // full-table kernel.  Off by default: on a B200 the two extra instructions per symbol cost more than the
     // added teams bring.
     const TensorDesc* hd = static_cast<const TensorDesc*>(c->h_descs.p);
-    pin_ensure(c->h_order, W * 4);
+    pin_ensure(c->h_order, 2 * W * 4);
     uint32_t* const order = static_cast<uint32_t*>(c->h_order.p);
     for (size_t i = 0; i < W; ++i) order[i] = (uint32_t)i;
     std::stable_sort(order, order + W, [&](uint32_t a, uint32_t b) { return hd[a].n_bytes > hd[b].n_bytes; });
@@ -919,12 +944,32 @@ static void run_decode(Context* c, size_t W, const uint8_t* d_payload, const uin
                            }) - order);
     bool any_int = false;
     for (size_t k = n_short; k < W && !any_int; ++k) any_int = hd[order[k]].spe * 2 != hd[order[k]].es;
+    // The kernel that keeps a chain's thread to its steps, or (short tensors, many integers, the options that only it
+    // has) the one that does everything in one thread.
+    size_t n_units = W, int_units = 0;
+    uint64_t rows = 0;
+    for (size_t i = 0; i < W; ++i) {
+        const bool ints = hd[i].spe * 2 != hd[i].es;
+        n_units += ints;
+        int_units += ints ? 2 : 0;
+        rows += (hd[i].n_bytes >> 8) * (ints ? 2 : 1);
+    }
+    const bool split = !n_short && !c->verify_zero_lanes && !c->decode_teams_per_sm &&
+                       prefer_split(n_units, int_units, rows, (size_t)(c->sm_count > 0 ? c->sm_count : 1));
+    if (split) {  // units: an integer tensor is two
+        size_t at = n_units;
+        for (size_t k = W; k-- > 0;) {  // from the end, in place
+            const uint32_t i = order[k];
+            if (hd[i].spe * 2 != hd[i].es) order[--at] = i | 0x80000000u;
+            order[--at] = i;
+        }
+    }
     dev_ensure(c, c->d_descs, W * sizeof(TensorDesc));
-    dev_ensure(c, c->d_order, W * 4);
+    dev_ensure(c, c->d_order, n_units * 4);
     dev_ensure(c, c->d_ticket, 256);
     ControlOps up;
     up.copy(c->d_descs.p, c->h_descs.p, W * sizeof(TensorDesc));
-    up.copy(c->d_order.p, order, W * 4);
+    up.copy(c->d_order.p, order, (split ? n_units : W) * 4);
     up.zero(c->d_ticket.p, 256);
     control_batch(c, up, s);
     CHK_CUDA(cudaEventRecord(c->ev[1], s));
@@ -939,13 +984,24 @@ static void run_decode(Context* c, size_t W, const uint8_t* d_payload, const uin
         c->launches++;
     };
     launch(rans_decode_kernel<false, true>, kDecSmemBytes[0][1], 0, n_short, 0);
-    // up to two teams an SM a scheduler has two warps at most, and a chain's latency is what counts (see dec_step)
     const size_t n = W - n_short;
-    const bool few = n <= 2 * (size_t)(c->sm_count > 0 ? c->sm_count : 1);
-    if (any_int)
-        launch(few ? rans_decode_kernel<true, false, true> : rans_decode_kernel<true, false, false>, kDecSmemBytes[1][0], n_short, n, 8);
-    else
-        launch(few ? rans_decode_kernel<false, false, true> : rans_decode_kernel<false, false, false>, kDecSmemBytes[0][0], n_short, n, 8);
+    if (split) {
+        SplitParams fp{};
+        fp.descs = static_cast<const TensorDesc*>(c->d_descs.p);
+        fp.cum_tables = d_cum;
+        fp.hdrs = d_hdrs;
+        fp.payload = d_payload;
+        fp.sidecar = d_sidecar;
+        fp.units = static_cast<const uint32_t*>(c->d_order.p);
+        fp.ticket = static_cast<uint32_t*>(c->d_ticket.p);
+        fp.n_units = (uint32_t)n_units;
+        fp.status = static_cast<uint32_t*>(c->h_status.p);
+        launch_split<0>(c, fp, s);
+    } else if (any_int) {
+        launch(rans_decode_kernel<true, false>, kDecSmemBytes[1][0], n_short, n, 8);
+    } else {
+        launch(rans_decode_kernel<false, false>, kDecSmemBytes[0][0], n_short, n, 8);
+    }
     CHK_CUDA(cudaEventRecord(c->ev[2], s));
     sync_stream(c, s);
     c->timing["decode_ms"] = ms_between(c->ev[1], c->ev[2]);

@@ -1217,7 +1217,7 @@ struct SlotTableSmem {
     uint32_t starts[kM / 32];         // bit s: a symbol's first slot
     uint16_t rank[kM / 32];           // starts before the word
     uint8_t present[256];             // symbols with slots, in order
-    uint32_t warp_tot[2][8];
+    uint32_t warp_tot[2][12];
 };
 // W = decoded lanes per 32-bit row word (2: float tensors only, 4: integers present)
 template <int W, bool ZS>
@@ -1235,6 +1235,14 @@ struct DecSmem {
 constexpr uint32_t kDecSmemBytes[2][2] = {{(uint32_t)sizeof(DecSmem<2, false>), (uint32_t)sizeof(DecSmem<2, true>)},
                                           {(uint32_t)sizeof(DecSmem<4, false>), (uint32_t)sizeof(DecSmem<4, true>)}};
 
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+#ifndef CHK_CPU_EMULATION
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+#else
+    (void)p;
+#endif
+}
+
 __device__ __forceinline__ uint32_t slot_entry(uint32_t sym, uint32_t f, uint32_t bias) { return sym | (bias << 8) | ((f - 1u) << 20); }
 
 // Slot table of one frequency table by kThreads threads (all of them; ends with a barrier).  A slot's symbol is the
@@ -1249,10 +1257,9 @@ __device__ __forceinline__ void build_slot_table(const uint32_t* __restrict__ cu
     __syncthreads();
     // symbols tid, tid + kThreads, ... that own slots: list and start bits
     uint32_t before = 0;
-    static_assert(256 % kThreads == 0, "every thread has a symbol in every round");
     for (uint32_t base = 0; base < 256; base += kThreads) {
         const uint32_t s = base + tid;
-        const bool has = b.cum[s + 1] > b.cum[s] && b.cum[s] < kM;  // (a damaged file's table may be anything)
+        const bool has = s < 256 && b.cum[s + 1] > b.cum[s] && b.cum[s] < kM;  // (a damaged file's table may be anything)
         const uint32_t m = __ballot_sync(0xffffffffu, has);
         if (lane == 0) b.warp_tot[0][warp] = (uint32_t)__popc(m);
         __syncthreads();
@@ -1404,10 +1411,10 @@ __device__ __forceinline__ uint32_t put_byte(uint32_t acc, uint32_t v, uint32_t 
 // branching.  Returns the table entry (symbol in its low byte).  With e >> 8 = (f - 1) * 4096 + (slot - cum) the new
 // state f * (x >> 12) + slot - cum is (f - 1) * ((x >> 12) - 4096) + (e >> 8) + (x >> 12): two shifts and a
 // multiply-add, nothing masked.  The byte count (0 for x >= 2^23, 1 for x >= 2^15, else 2; a valid state is never
-// below 2^11) comes from the leading zeros, which spares the integer pipe a full SM is bound by (31 cycles a step and
-// scheduler against 34), or -- kFew: a warp more or less alone on its scheduler -- from two comparisons, which are
-// sooner there (70 cycles a step against 82).
-template <bool ZS, bool kFew>
+// below 2^11) comes from the leading zeros: against two comparisons that spares the integer pipe a full SM is bound by
+// (31 cycles a step and scheduler instead of 34), though a warp alone on its scheduler waits longer for it (82
+// cycles a step instead of 70).
+template <bool ZS>
 __device__ __forceinline__ uint32_t dec_step(DecChain& c, DecWindow& w, const uint32_t* dtab, int s1) {
     const uint32_t slot = c.x & (kM - 1);
     const uint32_t xs = c.x >> kScaleBits;
@@ -1420,20 +1427,14 @@ __device__ __forceinline__ uint32_t dec_step(DecChain& c, DecWindow& w, const ui
         e = dtab[slot];
         x = (e >> 20) * (xs - 4096u) + ((e >> 8) + xs);
     }
-    uint32_t b;
-    if (kFew) {
-        b = x < (1u << 23) ? 8u : 0u;
-        b = x < (1u << 15) ? 16u : b;
-    } else {
-        b = ((uint32_t)__clz((int)x) - 1u) & 24u;
-    }
+    const uint32_t b = ((uint32_t)__clz((int)x) - 1u) & 24u;
     c.x = __funnelshift_l(w.hi, x, b);
     w.hi = __funnelshift_l(w.lo, w.hi, b);
     c.rel += b >> 3;
     return e;
 }
 
-template <int NV, int B0, bool ZS, bool kFew>
+template <int NV, int B0, bool ZS>
 __device__ __forceinline__ void decode_tensor(const TensorDesc& d, uint32_t ti, const uint32_t* __restrict__ cum_tables,
                                               const LaneHeader* __restrict__ hdrs, const uint8_t* __restrict__ payload,
                                               const uint8_t* __restrict__ sidecar, uint32_t check_zero_lanes,
@@ -1475,7 +1476,7 @@ __device__ __forceinline__ void decode_tensor(const TensorDesc& d, uint32_t ti, 
     };
     auto one = [&](int k) {  // a single symbol
         DecWindow w = dec_window(ch[k], ring[k]);
-        return dec_step<ZS, kFew>(ch[k], w, dtab, s1);
+        return dec_step<ZS>(ch[k], w, dtab, s1);
     };
 
     uint32_t r = 0;
@@ -1526,8 +1527,8 @@ __device__ __forceinline__ void decode_tensor(const TensorDesc& d, uint32_t ti, 
 #pragma unroll
                 for (int v = 0; v < 4; v += 2) {
                     DecWindow w = dec_window(ch[0], ring[0]);
-                    acc[q] = put_byte(acc[q], dec_step<ZS, kFew>(ch[0], w, dtab, s1), v);
-                    acc[q] = put_byte(acc[q], dec_step<ZS, kFew>(ch[0], w, dtab, s1), v + 1);
+                    acc[q] = put_byte(acc[q], dec_step<ZS>(ch[0], w, dtab, s1), v);
+                    acc[q] = put_byte(acc[q], dec_step<ZS>(ch[0], w, dtab, s1), v + 1);
                 }
                 if (q & 1) check_point();
             }
@@ -1580,7 +1581,7 @@ __device__ __forceinline__ void decode_tensor(const TensorDesc& d, uint32_t ti, 
                 for (int v = 0; v < 2; ++v) {
                     uint32_t e[2];
 #pragma unroll
-                    for (int k = 0; k < NV; ++k) e[k] = dec_step<ZS, kFew>(ch[k], w[k], dtab, s1);
+                    for (int k = 0; k < NV; ++k) e[k] = dec_step<ZS>(ch[k], w[k], dtab, s1);
                     store_pair(r + u + v, e[0], e[NV - 1]);
                 }
             }
@@ -1631,8 +1632,7 @@ __device__ __forceinline__ void decode_tensor(const TensorDesc& d, uint32_t ti, 
     __syncthreads();  // table and rings are reused by the next tensor
 }
 
-// One team per tensor.  kInts as for the encoder; ZS selects the table shape; kFew: so few tensors that a scheduler has
-// one warp or two (see dec_step).
+// One team per tensor.  kInts as for the encoder; ZS selects the table shape.
 #ifndef CHK_DEC_MINBLOCKS
 #define CHK_DEC_MINBLOCKS 8
 #endif
@@ -1642,8 +1642,8 @@ __device__ __forceinline__ void decode_tensor(const TensorDesc& d, uint32_t ti, 
 #ifndef CHK_DEC_ZS_MINBLOCKS
 #define CHK_DEC_ZS_MINBLOCKS 8
 #endif
-template <bool kInts, bool ZS, bool kFew = false>
-__global__ void __launch_bounds__(kTeam, ZS ? CHK_DEC_ZS_MINBLOCKS : kFew ? 2 : kInts ? CHK_DEC_INT_MINBLOCKS : CHK_DEC_MINBLOCKS) rans_decode_kernel(const TensorDesc* __restrict__ descs,
+template <bool kInts, bool ZS>
+__global__ void __launch_bounds__(kTeam, ZS ? CHK_DEC_ZS_MINBLOCKS : kInts ? CHK_DEC_INT_MINBLOCKS : CHK_DEC_MINBLOCKS) rans_decode_kernel(const TensorDesc* __restrict__ descs,
                                                             const uint32_t* __restrict__ freq_tables,  // [T][256]
                                                             const uint32_t* __restrict__ cum_tables,   // [T][257]
                                                             const LaneHeader* __restrict__ hdrs,
@@ -1671,11 +1671,11 @@ __global__ void __launch_bounds__(kTeam, ZS ? CHK_DEC_ZS_MINBLOCKS : kFew ? 2 : 
             continue;
         }
         if (d.es == 4 && d.spe == 2)
-            decode_tensor<1, 2, ZS, kFew>(d, ti, cum_tables, hdrs, payload, sidecar, check_zero_lanes, status, smem);
+            decode_tensor<1, 2, ZS>(d, ti, cum_tables, hdrs, payload, sidecar, check_zero_lanes, status, smem);
         else if (d.es == 2 && d.spe == 1)
-            decode_tensor<1, 1, ZS, kFew>(d, ti, cum_tables, hdrs, payload, sidecar, check_zero_lanes, status, smem);
+            decode_tensor<1, 1, ZS>(d, ti, cum_tables, hdrs, payload, sidecar, check_zero_lanes, status, smem);
         else if (kInts)
-            decode_tensor<2, 0, ZS, kFew>(d, ti, cum_tables, hdrs, payload, sidecar, check_zero_lanes, status, smem);
+            decode_tensor<2, 0, ZS>(d, ti, cum_tables, hdrs, payload, sidecar, check_zero_lanes, status, smem);
         else
             __syncthreads();
     }
@@ -1715,7 +1715,7 @@ struct PlaneDecSmem {
     SlotTableSmem build;
 };
 
-template <int kPlanes, bool kFew>
+template <int kPlanes>
 __device__ __forceinline__ void decode_plane_group(const PlaneGroup& g, const uint32_t* __restrict__ cum_tables,
                                                    const LaneHeader* __restrict__ hdrs,
                                                    const uint8_t* __restrict__ payload, uint32_t* __restrict__ status,
@@ -1778,7 +1778,7 @@ __device__ __forceinline__ void decode_plane_group(const PlaneGroup& g, const ui
 #pragma unroll
         for (int v = 0; v < 2; ++v)
 #pragma unroll
-            for (int k = 0; k < 2; ++k) acc = put_byte(acc, dec_step<false, kFew>(ch[k], w[k], dtab, 0), 2 * v + k);
+            for (int k = 0; k < 2; ++k) acc = put_byte(acc, dec_step<false>(ch[k], w[k], dtab, 0), 2 * v + k);
         return acc;
     };
     auto one_row = [&](uint32_t r, uint32_t limit) -> uint32_t {  // only the lanes below limit
@@ -1791,7 +1791,7 @@ __device__ __forceinline__ void decode_plane_group(const PlaneGroup& g, const ui
                 v = raw_col[((size_t)r << 8) + k];
             } else {
                 DecWindow w = dec_window(ch[k], ring[k]);
-                v = dec_step<false, kFew>(ch[k], w, dtab, 0) & 0xFFu;
+                v = dec_step<false>(ch[k], w, dtab, 0) & 0xFFu;
             }
             acc |= v << (8 * k);
         }
@@ -1877,7 +1877,7 @@ __device__ __forceinline__ void decode_plane_group(const PlaneGroup& g, const ui
     __syncthreads();  // tables and rings are reused by the next tensor
 }
 
-template <int kPlanes, bool kFew = false>
+template <int kPlanes>
 __global__ void __launch_bounds__(kPlanes * kTeam, kPlanes == 2 ? 2 : 5) rans_decode_planes_kernel(const PlaneGroup* __restrict__ groups,
                                                                             const uint32_t* __restrict__ cum_tables,
                                                                             const LaneHeader* __restrict__ hdrs,
@@ -1890,7 +1890,397 @@ __global__ void __launch_bounds__(kPlanes * kTeam, kPlanes == 2 ? 2 : 5) rans_de
     for (;;) {
         const uint32_t tk = next_ticket(ticket, &s_ticket);
         if (tk >= n_groups) break;
-        decode_plane_group<kPlanes, kFew>(groups[order[tk]], cum_tables, hdrs, payload, status, smem);
+        decode_plane_group<kPlanes>(groups[order[tk]], cum_tables, hdrs, payload, status, smem);
+    }
+}
+
+// ------------------------------------------------------------------ decode, steps and everything else in separate warps
+// The kernels above give a chain's thread everything: besides its step, moving blocks of the stream into the ring,
+// putting words together, the low bytes, the stores -- 32 instructions a row, and 145 cycles a row for a warp alone on
+// its scheduler, where the chain of dependent operations is 70 long.  Here that is the work of other warps.  A unit
+// is 128 chains (a float tensor's value lanes, or half the lanes of an integer tensor); four warps do nothing but
+// steps, 16 rows at a time, and leave their bytes and their read positions in shared memory; four helper warps, one
+// period behind, write those rows out and refill the rings.  One barrier per period, met by both sides' loops, which
+// run the same number of them.
+//   Rings hold four 32-byte blocks.  A helper that sees at most three unread after a period requests the next block
+// and stores it a period later, so it never waits for memory.  A period reads at most 32 bytes: the position seen leaves
+// at least 65 unread (at 97 and more nothing was requested a period before), the period that runs meanwhile leaves 33, and
+// the one in which the block is stored reads at most 32 of those.  The block that is replaced lies wholly behind the
+// position seen.
+//   128 tensors of 4 MiB (one unit an SM): 1.25 -> 0.69 ms, 83 cycles a row; 1024 tensors of 2 and 4 MiB (four units an
+// SM, the integer pipe two thirds busy): 3.13 -> 2.39 ms.
+// Units of container version 3 (kKind 1, 2) are half the lanes of the one or two byte planes of a tensor; with two
+// planes eight warps decode.
+constexpr uint32_t kSplitHelpers = 128;
+constexpr uint32_t kSplitRingBytes = 34 * 32 * 4;  // of a warp: 32 words a lane, and words 0 and 1 again behind word 31
+struct SplitParams {
+    const TensorDesc* descs;      // kKind 0
+    const PlaneGroup* groups;     // kKind 1, 2
+    const uint32_t* cum_tables;
+    const LaneHeader* hdrs;
+    const uint8_t* payload;
+    const uint8_t* sidecar;       // kKind 0
+    const uint32_t* units;        // index | part << 31, largest first
+    uint32_t* ticket;
+    uint32_t n_units;
+    uint32_t* status;
+};
+template <int kKind>
+struct SplitSmem {
+    static constexpr uint32_t kChains = kKind == 2 ? 256u : 128u;
+    uint32_t dtab[kKind == 2 ? 2 : 1][kM];
+    unsigned char ring[kChains / 32][kSplitRingBytes];
+    uint4 out[2][kChains];        // the bytes of a period's 16 rows, by chain
+    uint32_t pos[2][kChains];     // read positions after a period, in bits from the first block
+    SlotTableSmem build;
+};
+
+// One lane's stream as its helper sees it.
+struct SplitFeed {
+    const uint8_t* gp;    // next block
+    const uint8_t* gend;
+    uint32_t loaded;      // bytes in the ring so far, counted from the first block
+    uint8_t* ring;
+};
+__device__ __forceinline__ void split_put(SplitFeed& f, const uint4& a, const uint4& b) {
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint8_t* const at = f.ring + ((f.loaded & 96u) << 5);  // block (loaded / 32) & 3, eight words of 128 bytes
+#pragma unroll
+    for (int i = 0; i < 8; ++i) *reinterpret_cast<uint32_t*>(at + 128 * i) = __byte_perm(w[i], 0u, 0x0123);
+    if ((f.loaded & 96u) == 0) {
+        *reinterpret_cast<uint32_t*>(f.ring + 32 * 128) = __byte_perm(w[0], 0u, 0x0123);
+        *reinterpret_cast<uint32_t*>(f.ring + 33 * 128) = __byte_perm(w[1], 0u, 0x0123);
+    }
+    f.loaded += 32;
+    f.gp += 32;
+}
+
+// Requests a block if `take` (see dec_request), and starts the one behind it on its way to L2.
+__device__ __forceinline__ void split_load(uint32_t take, const uint8_t* gp, bool more, uint4& a, uint4& b) {
+#ifdef CHK_CPU_EMULATION
+    (void)more;
+    if (take) {
+        a = *reinterpret_cast<const uint4*>(gp);
+        b = *reinterpret_cast<const uint4*>(gp + 16);
+    }
+#else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %8, 0;\n\tsetp.ne.and.u32 q, %10, 0, p;\n\t"
+        "@p ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%9];\n\t@q prefetch.global.L2 [%9+32];\n\t}"
+        : "+r"(a.x), "+r"(a.y), "+r"(a.z), "+r"(a.w), "+r"(b.x), "+r"(b.y), "+r"(b.z), "+r"(b.w)
+        : "r"(take), "l"(gp), "r"(more ? 1u : 0u));
+#endif
+}
+// The block's barrier, from either side's loop.
+__device__ __forceinline__ void period_barrier() {
+#ifdef CHK_CPU_EMULATION
+    __syncthreads();
+#else
+    asm volatile("barrier.sync 0;" ::: "memory");
+#endif
+}
+
+template <int kKind>
+__device__ __forceinline__ void split_unit(const SplitParams& P, uint32_t unit, unsigned char* smem_raw) {
+    using Smem = SplitSmem<kKind>;
+    constexpr uint32_t kChains = Smem::kChains, kThreads = kChains + kSplitHelpers;
+    Smem* const sm = reinterpret_cast<Smem*>(smem_raw);
+    const uint32_t tid = threadIdx.x, part = unit >> 31, idx = unit & 0x7FFFFFFFu;
+    const bool stepping = tid < kChains;
+    const uint32_t h = stepping ? 0u : tid - kChains;  // helper number
+
+    // ---- what is decoded: rows of 256 bytes (kKind 0: of the tensor, else of a plane), and where it goes
+    TensorDesc d{};
+    PlaneGroup g{};
+    if (kKind == 0) d = P.descs[idx]; else g = P.groups[idx];
+    const unsigned long long B = kKind == 0 ? d.n_bytes : g.n_elem;
+    const bool floats = kKind == 0 && d.spe * 2 == d.es;
+    const uint32_t b0 = d.es == 4 ? 2u : 1u;  // lower value byte of a float tensor's word
+    const uint32_t full_rows = (uint32_t)(B >> 8), tail = (uint32_t)(B & 255), periods = full_rows / 16;
+    auto lane_of = [&](uint32_t c) -> uint32_t {  // lane of chain c
+        if (floats) return ((c >> 1) << 2) + ((c & 1u) ? 3u : b0);
+        return 128u * part + (c & 127u);
+    };
+    auto plane_of = [&](uint32_t c) -> uint32_t { return kKind == 2 ? c >> 7 : 0u; };
+    auto is_raw = [&](uint32_t c) { return kKind != 0 && g.plane[plane_of(c)].raw != 0; };
+    auto header = [&](uint32_t c) {
+        const size_t row = kKind == 0 ? idx : g.plane[plane_of(c)].hdr_index;
+        return P.hdrs[row * kLanes + lane_of(c)];
+    };
+    auto stream_at = [&](uint32_t c) { return kKind == 0 ? d.payload_off : g.plane[plane_of(c)].payload_off; };
+
+    // ---- start: helpers fill the rings, everybody builds the tables
+    uint32_t x = kL, pos = 0, pos_end = 0;  // a lane's stream is below 2^25 bytes
+    SplitFeed feed[kKind == 2 ? 2 : 1];
+    if (stepping) {
+        if (!is_raw(tid)) {
+            const LaneHeader lh = header(tid);
+            x = lh.final_state;
+            pos = (uint32_t)((stream_at(tid) + lh.buf_offset) & 31) * 8;
+            pos_end = pos + lh.byte_count * 8;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < kChains / kSplitHelpers; ++k) {
+            const uint32_t c = h + k * kSplitHelpers;
+            SplitFeed& f = feed[k];
+            f.ring = sm->ring[c >> 5] + (c & 31) * 4;
+            f.loaded = 0;
+            f.gp = f.gend = nullptr;
+            if (is_raw(c) || !(B > lane_of(c))) continue;  // nothing to read
+            const LaneHeader lh = header(c);
+            const unsigned long long p = stream_at(c) + lh.buf_offset;
+            f.gp = P.payload + (p & ~31ull);
+            // a valid stream needs nothing past its own end; one block more is read of a damaged one
+            f.gend = f.gp + (((((size_t)p & 31) + lh.byte_count + 31) & ~(size_t)31) + 32);
+            uint4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = f.gp + 32 * (i / 2) < f.gend ? ld_global_v4(f.gp + 16 * i) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) split_put(f, v[2 * i], v[2 * i + 1]);
+        }
+    }
+    if (kKind == 0) {
+        build_slot_table<kThreads>(P.cum_tables + (size_t)d.table_idx * 257, sm->build, tid, sm->dtab[0], 0u, 0u, kM);
+    } else {
+        for (int p = 0; p < kKind; ++p)
+            if (!g.plane[p].raw)
+                build_slot_table<kThreads>(P.cum_tables + (size_t)g.plane[p].table_idx * 257, sm->build, tid, sm->dtab[p], 0u, 0u, kM);
+        __syncthreads();
+    }
+    const uint32_t* const dtab = sm->dtab[stepping ? plane_of(tid) : 0u];
+    const uint8_t* const ring = stepping ? sm->ring[tid >> 5] + (tid & 31) * 4 : nullptr;
+    // The next eight stream bytes, first one on top: what four symbols can need at most.
+    auto window = [&]() {
+        const uint8_t* const at = ring + ((pos << 2) & 0xF80u);  // word (pos >> 5) & 31
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(at), w1 = *reinterpret_cast<const uint32_t*>(at + 128),
+                       w2 = *reinterpret_cast<const uint32_t*>(at + 256);
+        return DecWindow{__funnelshift_l(w1, w0, pos), __funnelshift_l(w2, w1, pos)};  // (shift counts are taken modulo 32)
+    };
+    auto step = [&](DecWindow& w) -> uint32_t {  // as dec_step; here the comparisons are sooner than the leading zeros
+        const uint32_t xs = x >> kScaleBits, e = dtab[x & (kM - 1)];
+        const uint32_t n = (e >> 20) * (xs - 4096u) + ((e >> 8) + xs);
+        uint32_t b = n < (1u << 23) ? 8u : 0u;
+        b = n < (1u << 15) ? 16u : b;
+        x = __funnelshift_l(w.hi, n, b);
+        w.hi = __funnelshift_l(w.lo, w.hi, b);
+        w.lo = __funnelshift_l(0u, w.lo, b);
+        pos += b;
+        return e;
+    };
+    // a plane stored raw is read instead
+    const bool raw = stepping && is_raw(tid);
+    const uint8_t* const raw_col = raw ? P.payload + stream_at(tid) + lane_of(tid) : nullptr;
+
+    // ---- what a helper writes of a period.  Its low bytes are requested a period ahead.
+    //   floats        word h >> 1 of the row, rows 8 (h & 1) .. + 7
+    //   integers      chains 4 (h & 31) .. + 3, rows 4 (h >> 5) .. + 3
+    //   one plane     the same chains and rows, two-byte elements
+    //   two planes    element h of the half row, all 16 rows
+    constexpr int kLow = kKind == 2 ? 16 : kKind == 1 ? 4 : 8;
+    const uint8_t* low_col = nullptr;
+    uint8_t* dst_col = nullptr;
+    bool low_ok = false, dst_ok = false;
+    uint32_t row0 = 0;
+    if (!stepping) {
+        if (floats) {
+            row0 = 8 * (h & 1);
+            low_col = P.sidecar + d.sidecar_off + 2 * (h >> 1);
+            dst_col = d.dst + 4 * (h >> 1);
+            low_ok = (reinterpret_cast<uintptr_t>(low_col) & 1) == 0;
+            dst_ok = (reinterpret_cast<uintptr_t>(dst_col) & 3) == 0;
+        } else if (kKind == 2) {
+            low_col = g.low + (128 * part + h) * 2;
+            dst_col = g.dst + (128 * part + h) * 4;
+            low_ok = (reinterpret_cast<uintptr_t>(low_col) & 1) == 0;
+            dst_ok = (reinterpret_cast<uintptr_t>(dst_col) & 3) == 0;
+        } else {
+            row0 = 4 * (h >> 5);
+            const uint32_t at = 128 * part + 4 * (h & 31);
+            low_col = kKind == 1 ? g.low + at : nullptr;
+            dst_col = kKind == 1 ? g.dst + at * 2 : d.dst + at;
+            low_ok = kKind == 0 || (reinterpret_cast<uintptr_t>(low_col) & 3) == 0;
+            dst_ok = (reinterpret_cast<uintptr_t>(dst_col) & (kKind == 1 ? 7 : 3)) == 0;
+        }
+    }
+    uint32_t low[kLow];
+    auto load_low = [&](uint32_t row, auto fast) {  // of rows row + row0 ...
+        if (kKind == 0 && !floats) return;
+        constexpr uint32_t kStride = kKind == 0 ? 128 : kKind == 1 ? 256 : 512;
+#pragma unroll
+        for (int u = 0; u < kLow; ++u) {
+            const uint8_t* p = low_col + (size_t)(row + row0 + u) * kStride;
+            if (kKind == 1)
+                low[u] = decltype(fast)::value ? *reinterpret_cast<const uint32_t*>(p)
+                                               : ((uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24));
+            else
+                low[u] = decltype(fast)::value ? (uint32_t)*reinterpret_cast<const uint16_t*>(p) : ((uint32_t)p[0] | ((uint32_t)p[1] << 8));
+        }
+        // the rows of two periods on start their way to L2
+        const uint32_t line = h * 128;
+        if (line < 16 * kStride && row + 48 <= full_rows) prefetch_l2((kKind == 0 ? P.sidecar + d.sidecar_off : g.low) + (size_t)(row + 32) * kStride + line);
+    };
+    auto put32 = [&](uint8_t* p, uint32_t w, auto fast) {
+        if (decltype(fast)::value) {
+            *reinterpret_cast<uint32_t*>(p) = w;
+        } else {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) p[b] = (uint8_t)(w >> (8 * b));
+        }
+    };
+    auto write_rows = [&](uint32_t row, const uint4* out, auto fast) {
+        if (floats) {
+            const uint2 lo = reinterpret_cast<const uint2*>(&out[h & ~1u])[h & 1], up = reinterpret_cast<const uint2*>(&out[h | 1u])[h & 1];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t v = u & 3;
+                const uint32_t pair = __byte_perm(u < 4 ? lo.x : lo.y, u < 4 ? up.x : up.y, v | ((4u + v) << 4));
+                put32(dst_col + ((size_t)(row + row0 + u) << 8), __byte_perm(low[u % kLow], pair, b0 == 2 ? 0x5410u : 0x5140u), fast);
+            }
+        } else if (kKind == 2) {
+            const uint4 p2 = out[h], p3 = out[(h + 128) % kChains];
+            const uint32_t a[4] = {p2.x, p2.y, p2.z, p2.w}, b[4] = {p3.x, p3.y, p3.z, p3.w};
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                const uint32_t v = u & 3;
+                put32(dst_col + (size_t)(row + u) * 1024,
+                      __byte_perm(low[u % kLow], __byte_perm(a[u >> 2], b[u >> 2], v | ((4u + v) << 4)), 0x5410u), fast);
+            }
+        } else {
+            uint32_t c[4], t[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) c[k] = reinterpret_cast<const uint32_t*>(&out[4 * (h & 31) + k])[h >> 5];
+            // 4 x 4 bytes: word k holds chain k's rows, word u shall hold row u's chains
+            const uint32_t l01 = __byte_perm(c[0], c[1], 0x5140), h01 = __byte_perm(c[0], c[1], 0x7362);
+            const uint32_t l23 = __byte_perm(c[2], c[3], 0x5140), h23 = __byte_perm(c[2], c[3], 0x7362);
+            t[0] = __byte_perm(l01, l23, 0x5410);
+            t[1] = __byte_perm(l01, l23, 0x7632);
+            t[2] = __byte_perm(h01, h23, 0x5410);
+            t[3] = __byte_perm(h01, h23, 0x7632);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                uint8_t* const p = dst_col + (size_t)(row + row0 + u) * (kKind == 1 ? 512 : 256);
+                if (kKind == 0) {
+                    put32(p, t[u], fast);
+                } else {
+                    const uint32_t e01 = __byte_perm(low[u % kLow], t[u], 0x5140), e23 = __byte_perm(low[u % kLow], t[u], 0x7362);
+                    if (decltype(fast)::value) {
+                        *reinterpret_cast<uint2*>(p) = make_uint2(e01, e23);
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {
+                            p[b] = (uint8_t)(e01 >> (8 * b));
+                            p[4 + b] = (uint8_t)(e23 >> (8 * b));
+                        }
+                    }
+                }
+            }
+        }
+    };
+
+    // ---- the periods, then what is left: helpers write the last rows, the others decode byte by byte
+    if (stepping) {
+        for (uint32_t p = 0; p < periods; ++p) {
+            uint32_t acc[4] = {0, 0, 0, 0};
+            if (!raw) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    DecWindow w = window();
+                    const uint32_t e0 = step(w), e1 = step(w), e2 = step(w), e3 = step(w);
+                    acc[q] = __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
+                }
+            } else {
+                const uint8_t* src = raw_col + ((size_t)p << 12);
+#pragma unroll
+                for (int u = 0; u < 16; ++u) acc[u >> 2] |= (uint32_t)src[u << 8] << (8 * (u & 3));
+            }
+            sm->out[p & 1][tid] = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+            sm->pos[p & 1][tid] = pos;
+            period_barrier();
+        }
+        const uint32_t t = lane_of(tid);
+        for (uint32_t r = periods * 16; r < full_rows + (t < tail ? 1u : 0u); ++r) {
+            uint32_t v;
+            if (raw) {
+                v = raw_col[(size_t)r << 8];
+            } else {
+                DecWindow w = window();
+                v = step(w);
+            }
+            const size_t at = ((size_t)r << 8) + t;
+            if (kKind == 0)
+                d.dst[at] = (uint8_t)v;
+            else if (kKind == 1)
+                g.dst[at * 2 + 1] = (uint8_t)v;
+            else
+                g.dst[at * 4 + 2 + plane_of(tid)] = (uint8_t)v;
+        }
+    } else {
+        auto loop = [&](auto fast) {
+            uint4 v[kKind == 2 ? 4 : 2] = {};  // blocks on their way
+            uint32_t take[kKind == 2 ? 2 : 1] = {};
+            for (uint32_t p = 0; p < periods; ++p) {
+#pragma unroll
+                for (uint32_t k = 0; k < kChains / kSplitHelpers; ++k) {
+                    SplitFeed& f = feed[k];
+                    if (take[k]) split_put(f, v[2 * k], v[2 * k + 1]);
+                    take[k] = p > 0 && f.gp < f.gend && f.loaded - (sm->pos[(p - 1) & 1][h + k * kSplitHelpers] >> 3) <= 96u;
+                    split_load(take[k], f.gp, f.gp + 32 < f.gend, v[2 * k], v[2 * k + 1]);
+                }
+                if (p > 0) write_rows((p - 1) * 16, sm->out[(p - 1) & 1], fast);
+                load_low(p * 16, fast);
+                period_barrier();
+            }
+            if (periods) write_rows((periods - 1) * 16, sm->out[(periods - 1) & 1], fast);
+        };
+        if (low_ok && dst_ok) loop(std::true_type{}); else loop(std::false_type{});
+        if (kKind != 0 || floats) {  // low bytes of the rows that are left
+            const uint32_t per = kKind == 0 ? d.spe : (uint32_t)kKind;  // low bytes of an element
+            const uint32_t es = kKind == 0 ? d.es : 2u * (uint32_t)kKind;
+            const unsigned long long n = kKind == 0 ? d.n_bytes / d.es : B;
+            const uint8_t* const src = kKind == 0 ? P.sidecar + d.sidecar_off : g.low;
+            uint8_t* const dst = kKind == 0 ? d.dst : g.dst;
+            const unsigned long long first = (unsigned long long)periods * 4096 / (kKind == 0 ? d.es : 1u) * per;
+            for (unsigned long long i = first + h; i < n * per; i += kSplitHelpers) {
+                if (kKind != 0 && part != (uint32_t)(((i / per) >> 7) & 1)) continue;  // the other half of the lanes: another unit
+                dst[i / per * es + i % per] = src[i];
+            }
+        }
+    }
+
+    if (stepping && !raw) {
+        uint32_t err = 0;
+        if (x != kL) err |= kErrEndState;
+        if (pos != pos_end) err |= kErrEndPointer;
+        if (err) atomicOr(&P.status[kKind == 0 ? idx : g.plane[plane_of(tid)].status_index], err);
+    }
+    __syncthreads();  // everything is reused by the next unit
+}
+
+template <int kKind>
+__global__ void __launch_bounds__(SplitSmem<kKind>::kChains + kSplitHelpers, kKind == 2 ? 2 : 4) rans_decode_split_kernel(const CHK_GRID_CONSTANT SplitParams P) {
+    CHK_DYN_SMEM(smem);
+    CHK_SHARED uint32_t s_ticket;
+    constexpr uint32_t kThreads = SplitSmem<kKind>::kChains + kSplitHelpers;
+    for (;;) {
+        const uint32_t tk = next_ticket(P.ticket, &s_ticket);
+        if (tk >= P.n_units) break;
+        const uint32_t unit = P.units[tk];
+        if (kKind == 0) {
+            const TensorDesc d = P.descs[unit & 0x7FFFFFFFu];
+            if (d.flags & kFlagRaw) {  // payload is the masked tensor
+                const uint8_t* in = P.payload + d.payload_off;
+                if (!(unit >> 31))
+                    for (unsigned long long i = threadIdx.x; i < d.n_bytes; i += kThreads) {
+                        const uint32_t jb = (uint32_t)(i % d.es);
+                        d.dst[i] = jb < d.spe ? P.sidecar[d.sidecar_off + (i / d.es) * d.spe + jb] : in[i];
+                    }
+                __syncthreads();  // s_ticket may be rewritten only after everyone has read it
+                continue;
+            }
+        }
+        split_unit<kKind>(P, unit, smem);
     }
 }
 

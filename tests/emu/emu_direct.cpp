@@ -75,4 +75,46 @@ void emu_block_sort(size_t n, const double* frac, int32_t* place_out) {
     for (size_t i = 0; i < n; ++i) place_out[i] = sm.place[i];
 }
 
+// rans_decode_split_kernel<0>: tensors.  rans_decode_split_kernel<1 or 2>: the planes of tensors, items numbered
+// [tensor * planes + plane].  Every part of every tensor is a unit; payload readable 64 bytes past its end, aligned.
+void emu_decode_split(size_t n, uint32_t planes, uint8_t* const* dsts, const uint64_t* n_bytes, const uint32_t* es, const uint32_t* spe,
+                    const uint8_t* const* lows, const uint32_t* cf, const uint32_t* hdrs, const uint8_t* payload,
+                    const uint64_t* payload_off, const uint8_t* raw, uint32_t* status_out, uint32_t grid) {
+    std::vector<TensorDesc> descs(n);
+    std::vector<PlaneGroup> groups(n);
+    std::vector<uint32_t> units;
+    for (size_t i = 0; i < n; ++i) {
+        TensorDesc& d = descs[i];
+        std::memset(&d, 0, sizeof(d));
+        d.dst = dsts[i];
+        d.n_bytes = n_bytes[i];
+        d.es = es[i];
+        d.spe = spe[i];
+        d.table_idx = (uint32_t)i;
+        d.payload_off = payload_off[i];
+        d.sidecar_off = planes ? 0 : (unsigned long long)(lows[i] - lows[0]);
+        if (raw[i]) d.flags |= kFlagRaw;
+        groups[i] = PlaneGroup{};
+        groups[i].dst = dsts[i];
+        groups[i].low = lows[i];
+        groups[i].n_elem = n_bytes[i];
+        for (uint32_t p = 0; p < planes; ++p) {
+            const uint32_t k = (uint32_t)(i * planes + p);
+            groups[i].plane[p] = PlaneItem{payload_off[k], k, k, raw[k], k};
+        }
+        units.push_back((uint32_t)i);
+        if (planes || spe[i] * 2 != es[i]) units.push_back((uint32_t)i | 0x80000000u);
+    }
+    std::memset(status_out, 0, n * (planes ? planes : 1) * 4);
+    uint32_t ticket = 0;
+    SplitParams fp{descs.data(), groups.data(), cf, (const LaneHeader*)hdrs, payload, planes ? nullptr : lows[0], units.data(), &ticket,
+                 (uint32_t)units.size(), status_out};
+    if (planes == 0)
+        emu::launch(grid, SplitSmem<0>::kChains + kSplitHelpers, sizeof(SplitSmem<0>), [&] { rans_decode_split_kernel<0>(fp); });
+    else if (planes == 1)
+        emu::launch(grid, SplitSmem<1>::kChains + kSplitHelpers, sizeof(SplitSmem<1>), [&] { rans_decode_split_kernel<1>(fp); });
+    else
+        emu::launch(grid, SplitSmem<2>::kChains + kSplitHelpers, sizeof(SplitSmem<2>), [&] { rans_decode_split_kernel<2>(fp); });
+}
+
 }  // extern "C"

@@ -126,6 +126,93 @@ def test_block_sort_leaves_the_order_of_std_sort(direct_lib, emu, n):
         assert np.array_equal(np.argsort(place), order), frac
 
 
+def _decode_split(lib, planes, dsts, n_bytes, es, spe, lows, cf, hdrs, payload, off, raw, grid=2):
+    n = len(dsts)
+    dp, lp = (C.c_void_p * n)(*[d.ctypes.data for d in dsts]), (C.c_void_p * n)(*[a.ctypes.data for a in lows])
+    a = [np.ascontiguousarray(v, t) for v, t in ((n_bytes, np.uint64), (es, np.uint32), (spe, np.uint32), (cf, np.uint32),
+                                                 (hdrs, np.uint32), (off, np.uint64), (raw, np.uint8))]
+    status = np.zeros(n * max(planes, 1), np.uint32)
+    padded = aligned(len(payload) + 128)
+    padded[:len(payload)] = payload
+    p = lambda v, t: v.ctypes.data_as(t)  # noqa: E731
+    lib.emu_decode_split(C.c_size_t(n), C.c_uint32(planes), dp, p(a[0], u64p), p(a[1], u32p), p(a[2], u32p), lp, p(a[3], u32p),
+                       p(a[4], u32p), p(padded, u8p), p(a[5], u64p), p(a[6], u8p), p(status, u32p), C.c_uint32(grid))
+    return status
+
+
+@pytest.mark.parametrize("kind", ["f32_master", "bf16_weight", "f32_exp_avg_sq_lognormal", "i8", "i32", "f32_uniform_bits"])
+@pytest.mark.parametrize("misalign", [0, 1, 2])
+def test_split_decode_of_tensors(direct_lib, oracle, kind, misalign):
+    """Sizes around rows and the 16-row periods; destinations and low bytes at odd addresses; a raw tensor; damage."""
+    es = ELEM_SIZE[synth(kind, 1, 0)[1]]
+    tensors = batch([(kind, max(1, b // es)) for b in EDGES + [11 * 4096 + 515]], [0])
+    masked, tabs = tables(oracle, tensors)
+    spe = SIDECAR_PER_ELEM[tensors[0][1]]
+    payloads, hdrs, raws, off, lows, dsts, around, at = [], [], [], [], [], [], [], 0
+    side = aligned(sum(a.size for a, _ in tensors) + 64)
+    lo = misalign
+    for i, ((a, dt), m, t) in enumerate(zip(tensors, masked, tabs)):
+        p, h, r = oracle.compress_tensor(m, *t[:3])
+        if i == 5:  # stored raw
+            p, h, r = m.copy(), np.zeros_like(h), True
+            h[0, 1] = m.size
+        payloads.append(p); hdrs.append(h); raws.append(r); off.append(at)
+        at += p.size
+        s = oracle.split(a, dt)[1] if spe else np.zeros(0, np.uint8)
+        side[lo:lo + s.size] = s
+        lows.append(side[lo:lo + 1])
+        lo += s.size
+        m0 = misalign * (es if es > 1 else 1)
+        d = aligned(a.size + 48)
+        d[:] = 0xEE
+        around.append((d, 16 + m0))
+        dsts.append(d[16 + m0:16 + m0 + a.size])
+    payload = np.concatenate(payloads)
+    args = ([a.size for a, _ in tensors], [es] * len(tensors), [spe] * len(tensors), lows, np.concatenate([t[1] for t in tabs]),
+            np.concatenate(hdrs))
+    status = _decode_split(direct_lib, 0, dsts, *args, payload, off, raws)
+    assert not status.any()
+    for d, (a, _), (whole, at0) in zip(dsts, tensors, around):
+        assert np.array_equal(d, a)
+        assert np.all(whole[:at0] == 0xEE) and np.all(whole[at0 + a.size:] == 0xEE)  # and nothing around it
+    if kind == "f32_master":
+        bad = payload.copy()
+        bad[off[9] + int(hdrs[9][3, 2]) + 1] ^= 0x55  # lane 3: a value lane
+        assert _decode_split(direct_lib, 0, dsts, *args, bad, off, raws)[9] != 0
+
+
+@pytest.mark.parametrize("kind,es", [("f32_master", 4), ("bf16_weight", 2), ("f32_exp_avg_sq_lognormal", 4)])
+@pytest.mark.parametrize("misalign", [0, 1])
+def test_split_decode_of_planes(direct_lib, oracle, kind, es, misalign):
+    rng = np.random.default_rng(3)
+    planes, sizes = es // 2, [8 * 4096 + 5 * 256 + 77, 4096, 255, 1, 256 * 9, 16 * 4096 + 128]
+    dsts, lows, want, n_elem, poff, raws, cfs, hdrs, payloads, at = [], [], [], [], [], [], [], [], [], 0
+    for gi, n in enumerate(sizes):
+        m = synth(kind, n, 70 + gi)[0].reshape(n, es).copy()
+        if gi == 1:
+            flat = np.tile(np.arange(256, dtype=np.uint8), n // 256)  # every value equally often: stored raw
+            rng.shuffle(flat)
+            m[:, es - 2 if planes == 2 else es - 1] = flat
+        want.append(m.reshape(-1).copy())
+        low = aligned(n * (es // 2) + 32)[misalign:misalign + n * (es // 2)]
+        low[:] = m[:, :es // 2].reshape(-1)
+        lows.append(low)
+        dsts.append(aligned(n * es + 32)[misalign * es:misalign * es + n * es])
+        n_elem.append(n)
+        for p in range(planes):
+            plane = np.ascontiguousarray(m[:, es // 2 + p])
+            nf, cf, xm, _ = oracle.normalize(oracle.byte_histogram(plane), False)
+            pay, h, is_raw = oracle.compress_tensor(plane, nf, cf, xm)
+            poff.append(at); raws.append(int(is_raw)); cfs.append(cf); hdrs.append(h); payloads.append(pay)
+            at += pay.size
+    assert any(raws)
+    status = _decode_split(direct_lib, planes, dsts, n_elem, [es] * len(sizes), [es // 2] * len(sizes), lows, np.concatenate(cfs),
+                         np.concatenate(hdrs), np.concatenate(payloads), poff, raws)
+    assert not status.any()
+    for d, w in zip(dsts, want):
+        assert np.array_equal(d, w)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("workspace", [0, 1 << 20])
 def test_files_on_the_device(oracle, tmp_path, workspace):
