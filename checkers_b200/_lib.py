@@ -29,7 +29,7 @@ def _load():
         raise ImportError(f"{LIB} is missing: build it with `python -m checkers_b200.build` "
                           "(nvcc, sm_100a). There is no CPU fallback.")
     lib = C.CDLL(LIB)
-    vp, u64, u32p, f32p = C.c_void_p, C.c_uint64, C.POINTER(C.c_uint32), C.POINTER(C.c_float)
+    vp, u64, u32p = C.c_void_p, C.c_uint64, C.POINTER(C.c_uint32)
     sig = {
         "chk_last_error": (C.c_char_p, []),
         "chk_context_create": (C.c_int, [C.c_int, C.c_int, C.c_int, C.POINTER(vp)]),
@@ -48,7 +48,7 @@ def _load():
         "chk_hll_merge": (C.c_int, [C.POINTER(C.c_uint8), C.POINTER(C.c_uint8)]),
         "chk_hll_count": (C.c_int, [C.POINTER(C.c_uint8), C.POINTER(C.c_double)]),
         "chk_shared_vocabulary_report": (C.c_int, [vp, C.POINTER(u64), C.POINTER(u64)]),
-        "chk_get_tensor_stats": (C.c_int, [vp, u64, u32p, f32p, f32p, f32p]),
+        "chk_get_tensor_stats": (C.c_int, [vp, u64, vp, vp, vp, vp]),
         "chk_get_cluster_ids": (C.c_int, [vp, C.POINTER(C.c_int32), u64, C.POINTER(C.c_int32)]),
         "chk_get_cluster_anchor": (C.c_int, [vp, C.c_int32, C.c_char_p]),
         "chk_set_cluster_info": (C.c_int, [vp, u64, C.POINTER(C.c_char_p), C.POINTER(C.c_int32), C.c_int32,

@@ -44,6 +44,7 @@ class Context:
         self.device, self.rank = int(device), int(rank)
         self._keep = []
         self.names = []
+        self._stats = None
 
     def close(self):
         if self._h:
@@ -122,12 +123,15 @@ class Context:
         return a.value, b.value
 
     def tensor_stats(self, index):
-        hist = np.zeros(256, np.uint32)
-        mom, mm, fp = np.zeros(4, np.float32), np.zeros(2, np.float32), np.zeros(5, np.float32)
-        f32p = C.POINTER(C.c_float)
-        check(lib.chk_get_tensor_stats(self._h, int(index), hist.ctypes.data_as(C.POINTER(C.c_uint32)),
-                                       mom.ctypes.data_as(f32p), mm.ctypes.data_as(f32p), fp.ctypes.data_as(f32p)))
-        return hist, mom, mm, fp
+        # the four results land in one scratch array whose addresses are made once: callers ask for thousands in a row
+        if self._stats is None:
+            buf = np.empty(267, np.uint32)
+            self._stats = (buf, *(C.c_void_p(buf.ctypes.data + o) for o in (0, 1024, 1040, 1048)))
+        buf, hist, moments, minmax, fingerprint = self._stats
+        check(lib.chk_get_tensor_stats(self._h, int(index), hist, moments, minmax, fingerprint))
+        out = buf.copy()
+        f = out.view(np.float32)
+        return out[:256], f[256:260], f[260:262], f[262:]
 
     def cluster_ids(self):
         n = self.tensor_count()

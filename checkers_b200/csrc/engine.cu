@@ -1238,13 +1238,43 @@ static void analyze(Context* c) {
         const Tensor& t = c->tensors[i];
         d[i] = StatsDesc{elem_size(t.dtype) ? t.ptr : nullptr, t.n_elem, t.dtype, c->histogram_bins};
     }
+    // In the reference's order a tensor is one block, or -- when there are too few tensors to fill the device that way,
+    // or one of them is longer than an SM's share of all -- eight one-warp blocks.  Eight blocks of 256 threads an SM is
+    // where the one-block kernel reaches its bandwidth (4.95 TB/s at 26 tensors an SM).
+    const size_t sms = (size_t)(c->sm_count > 0 ? c->sm_count : 1);
+    uint64_t all = 0, longest = 0;
+    for (size_t i = 0; i < N; ++i) {
+        all += d[i].n;
+        longest = std::max<uint64_t>(longest, d[i].n);
+    }
+    const bool slices = !c->fast_stats && (N < 8 * sms || longest > all / sms);
     dev_ensure(c, c->d_stats_desc, N * sizeof(StatsDesc));
     dev_ensure(c, c->d_stats_out, N * sizeof(StatsOut));
-    pin_ensure(c->h_stats, N * sizeof(StatsOut));
-    CHK_CUDA(cudaMemcpyAsync(c->d_stats_desc.p, d.data(), N * sizeof(StatsDesc), cudaMemcpyHostToDevice, s));
-    CHK_CUDA(cudaMemsetAsync(c->d_stats_out.p, 0, N * sizeof(StatsOut), s));
+    pin_ensure(c->h_stats, N * (sizeof(StatsOut) + sizeof(StatsDesc)));
+    StatsDesc* const h_desc = reinterpret_cast<StatsDesc*>(static_cast<StatsOut*>(c->h_stats.p) + N);
+    std::memcpy(h_desc, d.data(), N * sizeof(StatsDesc));
+    SliceParams sp{};
+    ControlOps up;
+    up.copy(c->d_stats_desc.p, h_desc, N * sizeof(StatsDesc));
+    up.zero(c->d_stats_out.p, N * sizeof(StatsOut));
+    if (slices) {
+        dev_ensure(c, c->d_stats_part, N * (2 * 768 + 1) * 4);
+        sp.descs = static_cast<const StatsDesc*>(c->d_stats_desc.p);
+        sp.outs = static_cast<StatsOut*>(c->d_stats_out.p);
+        sp.part1 = static_cast<float*>(c->d_stats_part.p);
+        sp.part2 = sp.part1 + N * 768;
+        sp.done = reinterpret_cast<uint32_t*>(sp.part2 + N * 768);
+        sp.n_tensors = (uint32_t)N;
+        up.zero(sp.done, N * 4);
+    }
+    control_batch(c, up, s);
     CHK_CUDA(cudaEventRecord(c->ev[0], s));
-    if (!c->fast_stats) {
+    if (slices) {
+        stats_slices1_kernel<<<(uint32_t)(N * kSlices), 32, 0, s>>>(sp);
+        stats_slices2_kernel<<<(uint32_t)(N * kSlices), 32, 0, s>>>(sp);
+        CHK_CUDA(cudaGetLastError());
+        c->launches += 2;
+    } else if (!c->fast_stats) {
         const size_t cap = (size_t)(c->sm_count > 0 ? c->sm_count : 1) * 64;
         const uint32_t grid = (uint32_t)(N < cap ? N : cap);
         tensor_stats_kernel<<<grid, 256, 0, s>>>(static_cast<const StatsDesc*>(c->d_stats_desc.p),
@@ -1284,7 +1314,7 @@ static void analyze(Context* c) {
         }
     }
     CHK_CUDA(cudaEventRecord(c->ev[1], s));
-    CHK_CUDA(cudaMemcpyAsync(c->h_stats.p, c->d_stats_out.p, N * sizeof(StatsOut), cudaMemcpyDeviceToHost, s));
+    control_copy(c, c->h_stats.p, c->d_stats_out.p, N * sizeof(StatsOut), s);
     sync_stream(c, s);
     c->timing["analyze_stats_ms"] = ms_between(c->ev[0], c->ev[1]);
     std::memcpy(c->stats.data(), c->h_stats.p, N * sizeof(StatsOut));

@@ -347,4 +347,201 @@ __global__ void __launch_bounds__(256) stats_fast_reduce2_kernel(const StatsDesc
     }
 }
 
+// ------------------------------------------------------------------ the reference's order over more of the device
+// tensor_stats_kernel keeps a tensor on one block, so a batch of few or very unequal tensors leaves most SMs idle
+// (128 tensors of up to 16 MB: 3.9 ms, 15 % of the copy rate).  The 256 strided chains of a tensor are independent
+// until the halving tree, so here a warp takes 32 of them: eight one-warp blocks per tensor, up to 2 kSliceAhead loads
+// of a thread in flight.  The tree is the same: every block of the second pass rebuilds it from the first
+// pass' 256 partials (three steps inside a thread, five across the warp), and the block that finishes a tensor last
+// (a counter that starts at zero; nobody waits) combines the second pass' partials.  Same additions in the same
+// order, so the same bits.
+constexpr uint32_t kSlices = 8;       // blocks per tensor
+constexpr int kSliceAhead = 32;
+
+struct SliceParams {
+    const StatsDesc* descs;
+    StatsOut* outs;        // zeroed
+    float* part1;          // [n][3][256]: minimum, maximum, sum of every chain
+    float* part2;          // [n][3][256]: second, third, fourth central powers
+    uint32_t* done;        // [n], zeroed
+    uint32_t n_tensors;
+};
+
+template <int DT>
+__device__ __forceinline__ float slice_value(const void* p, unsigned long long i) {
+#ifndef CHK_CPU_EMULATION
+    if (DT == 2) {
+        float f;
+        asm("cvt.f32.f16 %0, %1;" : "=f"(f) : "h"(reinterpret_cast<const uint16_t*>(p)[i]));
+        return f;
+    }
+#endif
+    return load_value_t<DT>(p, i);
+}
+
+// f(element) for elements t, t + 256, ... of n, in order.  Two batches of kSliceAhead loads alternate, each loaded as a
+// whole while the other is used: a register loaded again right after its use would leave the hardware waiting for the
+// newest of the loads that share its scoreboard (8.2 ms instead of 3.9 before).
+template <int DT, typename F>
+__device__ __forceinline__ void slice_for_each(const void* p, unsigned long long n, uint32_t t, F&& f) {
+    constexpr unsigned long long kBatch = (unsigned long long)kSliceAhead * 256;
+    unsigned long long i = t;
+    unsigned long long left = (n > t ? (n - t + 255) / 256 : 0) / kSliceAhead;  // whole batches not used yet
+    auto load = [&](float (&v)[kSliceAhead], unsigned long long at) {
+#pragma unroll
+        for (int k = 0; k < kSliceAhead; ++k) v[k] = slice_value<DT>(p, at + (unsigned long long)k * 256);
+    };
+    auto use = [&](const float (&v)[kSliceAhead]) {
+#pragma unroll
+        for (int k = 0; k < kSliceAhead; ++k) f(v[k]);
+    };
+    if (left) {
+        float a[kSliceAhead], b[kSliceAhead];
+        load(a, i);  // the first of the batches that are left is in a
+        for (; left > 2; left -= 2) {
+            load(b, i + kBatch);
+            use(a);
+            load(a, i + 2 * kBatch);
+            use(b);
+            i += 2 * kBatch;
+        }
+        if (left == 2) {
+            load(b, i + kBatch);
+            use(a);
+            use(b);
+        } else {
+            use(a);
+        }
+        i += left * kBatch;
+    }
+    // less than a batch
+    if (i < n) {
+        float v[kSliceAhead];
+#pragma unroll
+        for (int k = 0; k < kSliceAhead; ++k) v[k] = i + (unsigned long long)k * 256 < n ? slice_value<DT>(p, i + (unsigned long long)k * 256) : 0.0f;
+#pragma unroll
+        for (int k = 0; k < kSliceAhead; ++k)
+            if (i + (unsigned long long)k * 256 < n) f(v[k]);
+    }
+}
+template <typename F>
+__device__ __forceinline__ void slice_dispatch(const StatsDesc& d, uint32_t t, F&& f) {
+    switch (d.dtype) {
+        case 0: slice_for_each<0>(d.ptr, d.n, t, f); break;
+        case 1: slice_for_each<1>(d.ptr, d.n, t, f); break;
+        case 2: slice_for_each<2>(d.ptr, d.n, t, f); break;
+        case 3: slice_for_each<3>(d.ptr, d.n, t, f); break;
+        default: slice_for_each<4>(d.ptr, d.n, t, f); break;
+    }
+}
+
+// The halving tree over 256 partials by one warp: thread l holds partials l, l + 32, ..., so the steps 128, 64, 32 are its own.
+template <typename Op>
+__device__ __forceinline__ float slice_tree(const volatile float* part, uint32_t lane, Op&& op) {
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = part[32 * k + lane];
+#pragma unroll
+    for (int s = 4; s > 0; s >>= 1)
+#pragma unroll
+        for (int k = 0; k < s; ++k) v[k] = op(v[k], v[k + s]);
+    float r = v[0];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) r = op(r, __shfl_xor_sync(0xffffffffu, r, s));  // lanes below s hold what the tree holds
+    return __shfl_sync(0xffffffffu, r, 0);
+}
+
+__global__ void __launch_bounds__(32) stats_slices1_kernel(const SliceParams P) {
+    const uint32_t ti = blockIdx.x / kSlices, t = (blockIdx.x % kSlices) * 32 + threadIdx.x;
+    if (ti >= P.n_tensors) return;
+    const StatsDesc d = P.descs[ti];
+    if (!d.ptr || d.n == 0 || d.dtype > 4u) return;
+    float lo = 1e37f, hi = -1e37f, sum = 0.0f;
+    slice_dispatch(d, t, [&](float x) {
+        lo = fminf(lo, x);
+        hi = fmaxf(hi, x);
+        sum = __fadd_rn(sum, x);
+    });
+    float* const out = P.part1 + (size_t)ti * 768;
+    out[t] = lo;
+    out[256 + t] = hi;
+    out[512 + t] = sum;
+}
+
+__global__ void __launch_bounds__(32) stats_slices2_kernel(const SliceParams P) {
+    CHK_SHARED uint32_t wh[256];
+    const uint32_t ti = blockIdx.x / kSlices, lane = threadIdx.x, t = (blockIdx.x % kSlices) * 32 + lane;
+    if (ti >= P.n_tensors) return;
+    const StatsDesc d = P.descs[ti];
+    if (!d.ptr || d.n == 0 || d.dtype > 4u) return;
+    StatsOut& o = P.outs[ti];
+    const int bins = (int)(d.bins < 256u ? d.bins : 256u);
+    for (uint32_t k = lane; k < 256; k += 32) wh[k] = 0;
+    const float* const p1 = P.part1 + (size_t)ti * 768;
+    const auto add = [](float a, float b) { return __fadd_rn(a, b); };
+    const float vmin = slice_tree(p1, lane, [](float a, float b) { return fminf(a, b); });
+    const float vmax = slice_tree(p1 + 256, lane, [](float a, float b) { return fmaxf(a, b); });
+    const float nf = (float)d.n;
+    const float mean = __fdiv_rn(slice_tree(p1 + 512, lane, add), nf);
+    const float range = __fsub_rn(vmax, vmin);
+    const bool wide = range > 1e-9f;
+    const float scale = wide ? __fdiv_rn(__fsub_rn((float)bins, 1.0f), range) : 0.0f;
+    warp_fence();
+
+    // One shared-memory increment per value: lanes that hit one counter are merged by the hardware, which beats runs of
+    // equal bins kept in registers (1.33 -> 1.01 ms).  Nothing in here branches, so the elements of a batch overlap: with
+    // the two tests that stats_bin makes per element the pass took 190 cycles an element.  (Too narrow a range for bins
+    // has scale 0, which puts every value into bin 0 all the same; and no value is below the minimum, so no bin is
+    // negative.)
+    float m2 = 0.0f, m3 = 0.0f, m4 = 0.0f;
+    const uint32_t top = bins > 0 ? (uint32_t)bins - 1u : 0u;
+    auto element = [&](float x, auto counted) {
+        const float from_min = __fsub_rn(x, vmin);
+        if (decltype(counted)::value) {
+            const uint32_t b = (uint32_t)(int)__fmul_rn(from_min, scale);
+            atomicAdd(&wh[b < top ? b : top], 1u);
+        }
+        const float dd = __fsub_rn(x, mean);
+        const float d2 = __fmul_rn(dd, dd);
+        m2 = __fadd_rn(m2, d2);
+        m3 = __fadd_rn(m3, __fmul_rn(d2, dd));
+        m4 = __fadd_rn(m4, __fmul_rn(d2, d2));
+    };
+    if (bins > 0)
+        slice_dispatch(d, t, [&](float x) { element(x, std::true_type{}); });
+    else
+        slice_dispatch(d, t, [&](float x) { element(x, std::false_type{}); });
+    warp_fence();
+    for (uint32_t k = lane; k < 256; k += 32) {
+        const uint32_t c = *(volatile uint32_t*)&wh[k];
+        if (c) atomicAdd(&o.hist[k], c);
+    }
+    float* const p2 = P.part2 + (size_t)ti * 768;
+    p2[t] = m2;
+    p2[256 + t] = m3;
+    p2[512 + t] = m4;
+    __threadfence();
+    warp_fence();
+    uint32_t before = 0;
+    if (lane == 0) before = atomicAdd(&P.done[ti], 1u);
+    if (__shfl_sync(0xffffffffu, before, 0) + 1u != kSlices) return;
+    __threadfence();
+    const float M2 = __fdiv_rn(slice_tree(p2, lane, add), nf), M3 = __fdiv_rn(slice_tree(p2 + 256, lane, add), nf),
+                M4 = __fdiv_rn(slice_tree(p2 + 512, lane, add), nf);
+    if (lane) return;
+    float skew = 0.0f, kurt = 0.0f;
+    if (M2 > 1e-9f) {
+        const float sd = __fsqrt_rn(M2);
+        skew = __fdiv_rn(M3, __fmul_rn(M2, sd));
+        kurt = __fdiv_rn(M4, __fmul_rn(M2, M2));
+    }
+    o.moments[0] = o.fingerprint[0] = mean;
+    o.moments[1] = o.fingerprint[1] = M2;
+    o.moments[2] = o.fingerprint[2] = skew;
+    o.moments[3] = o.fingerprint[3] = kurt;
+    o.minmax[0] = vmin;
+    o.minmax[1] = vmax;
+    o.fingerprint[4] = range;
+}
+
 }  // namespace chk
