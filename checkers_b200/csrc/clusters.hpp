@@ -9,10 +9,14 @@
 // handed out in category-name order, then by union-find root.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstdint>
+#include <cstring>
 #include <map>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -31,6 +35,45 @@ inline const char* category_of_name(const std::string& name) {
     return "model_state";
 }
 
+// f(0 .. n-1), on a few threads when the work is worth their start (tens of microseconds each).
+template <typename F>
+inline void cluster_parallel(size_t n, size_t work, F&& f) {
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t threads = std::min(std::min<size_t>(n, hw), std::min<size_t>(8, work / 50000 + 1));
+    if (threads <= 1) {
+        for (size_t i = 0; i < n; ++i) f(i);
+        return;
+    }
+    std::atomic<size_t> next{0};
+    auto run = [&] {
+        for (size_t i; (i = next.fetch_add(1)) < n;) f(i);
+    };
+    std::vector<std::thread> pool;
+    for (size_t k = 1; k < threads; ++k) pool.emplace_back(run);
+    run();
+    for (auto& t : pool) t.join();
+}
+
+// The element that sorting v (none negative) would leave at position `at`.  Doubles that are not negative order like
+// their bits: count the leading 16, then select inside the one bucket that holds the position.
+inline double cluster_select(const std::vector<double>& v, size_t at) {
+    std::vector<uint32_t> bucket(65536, 0);
+    auto top = [](double x) {
+        uint64_t b;
+        std::memcpy(&b, &x, 8);
+        return (size_t)(b >> 48);
+    };
+    for (double x : v) ++bucket[top(x)];
+    size_t k = 0, before = 0;
+    while (before + bucket[k] <= at) before += bucket[k++];
+    std::vector<double> in;
+    in.reserve(bucket[k]);
+    for (double x : v)
+        if (top(x) == k) in.push_back(x);
+    std::nth_element(in.begin(), in.begin() + (at - before), in.end());
+    return in[at - before];
+}
+
 // fingerprints: 5 floats per tensor {mean, variance, skewness, kurtosis, range}
 inline ClusterMap build_clusters(const std::vector<std::string>& names, const std::vector<float>& fingerprints) {
     ClusterMap out;
@@ -42,62 +85,112 @@ inline ClusterMap build_clusters(const std::vector<std::string>& names, const st
         std::vector<int> parent, rank;
         explicit DisjointSet(int m) : parent(m), rank(m, 0) { std::iota(parent.begin(), parent.end(), 0); }
         int find(int v) { return parent[v] == v ? v : parent[v] = find(parent[v]); }
-        void unite(int a, int b) {
+        int unite(int a, int b) {  // how many sets fewer
             a = find(a);
             b = find(b);
-            if (a == b) return;
+            if (a == b) return 0;
             if (rank[a] < rank[b]) std::swap(a, b);
             parent[b] = a;
             if (rank[a] == rank[b]) ++rank[a];
+            return 1;
         }
     };
 
+    // Of every category: the coordinates by dimension, and the squared distances of its pairs (a, b > a), row by row.
+    struct Category {
+        const std::vector<size_t>* idx;
+        int m;
+        double spread[5];
+        std::vector<double> at[5], squared;
+        std::vector<int> root;
+        bool usable = true;
+    };
+    std::vector<Category> cats;
+    size_t pairs = 0;
+    struct RowBlock {
+        size_t cat;
+        int first, last;
+    };
+    std::vector<RowBlock> blocks;
     for (const auto& entry : groups) {
-        const std::vector<size_t>& idx = entry.second;
-        const int m = (int)idx.size();
-        if (m == 0) continue;
-        auto val = [&](int a, int k) { return (double)fingerprints[idx[a] * 5 + k]; };
-
-        double mean[5] = {}, spread[5] = {};
-        for (int a = 0; a < m; ++a)
-            for (int k = 0; k < 5; ++k) mean[k] += val(a, k);
-        for (int k = 0; k < 5; ++k) mean[k] /= m;
-        for (int a = 0; a < m; ++a)
-            for (int k = 0; k < 5; ++k) {
-                const double dv = val(a, k) - mean[k];
-                spread[k] += dv * dv;
+        Category c;
+        c.idx = &entry.second;
+        const int m = c.m = (int)entry.second.size();
+        double mean[5] = {};
+        for (int k = 0; k < 5; ++k) {
+            c.at[k].resize(m);
+            c.spread[k] = 0;
+            for (int a = 0; a < m; ++a) {
+                c.at[k][a] = (double)fingerprints[entry.second[a] * 5 + k];
+                mean[k] += c.at[k][a];
             }
-        for (int k = 0; k < 5; ++k) spread[k] = (spread[k] / m < 1e-30) ? 1.0 : std::sqrt(spread[k] / m);
-
-        auto distance = [&](int a, int b) {
-            double acc = 0;
-            for (int k = 0; k < 5; ++k) {
-                const double dv = (val(a, k) - val(b, k)) / spread[k];
-                acc += dv * dv;
+            mean[k] /= m;
+            for (int a = 0; a < m; ++a) {
+                const double dv = c.at[k][a] - mean[k];
+                c.spread[k] += dv * dv;
             }
-            return std::sqrt(acc);
-        };
-
-        std::vector<double> pairwise;
-        pairwise.reserve((size_t)m * (m - 1) / 2);
-        for (int a = 0; a < m; ++a)
-            for (int b = a + 1; b < m; ++b) pairwise.push_back(distance(a, b));
-        double threshold = 0.0;
-        if (!pairwise.empty()) {
-            // the reference sorts all distances and takes element size/4; that order statistic is all it uses
-            std::vector<double> sorted = pairwise;
-            std::nth_element(sorted.begin(), sorted.begin() + sorted.size() / 4, sorted.end());
-            threshold = sorted[sorted.size() / 4];
+            c.spread[k] = (c.spread[k] / m < 1e-30) ? 1.0 : std::sqrt(c.spread[k] / m);
         }
+        c.squared.resize((size_t)m * (m - 1) / 2);
+        pairs += c.squared.size();
+        for (int a = 0; a < m; a += 32) blocks.push_back(RowBlock{cats.size(), a, std::min(a + 32, m)});
+        cats.push_back(std::move(c));
+    }
 
-        DisjointSet ds(m);
-        size_t p = 0;
-        for (int a = 0; a < m; ++a)
-            for (int b = a + 1; b < m; ++b, ++p)
-                if (pairwise[p] < threshold) ds.unite(a, b);
+    cluster_parallel(blocks.size(), pairs, [&](size_t i) {
+        const RowBlock& r = blocks[i];
+        Category& c = cats[r.cat];
+        const double* const p[5] = {c.at[0].data(), c.at[1].data(), c.at[2].data(), c.at[3].data(), c.at[4].data()};
+        const double s0 = c.spread[0], s1 = c.spread[1], s2 = c.spread[2], s3 = c.spread[3], s4 = c.spread[4];
+        for (int a = r.first; a < r.last; ++a) {
+            double* const out_row = c.squared.data() + ((size_t)a * (2 * (size_t)c.m - a - 1)) / 2 - (a + 1);
+            const double x0 = p[0][a], x1 = p[1][a], x2 = p[2][a], x3 = p[3][a], x4 = p[4][a];
+            for (int b = a + 1; b < c.m; ++b) {
+                const double d0 = (x0 - p[0][b]) / s0, d1 = (x1 - p[1][b]) / s1, d2 = (x2 - p[2][b]) / s2,
+                             d3 = (x3 - p[3][b]) / s3, d4 = (x4 - p[4][b]) / s4;
+                out_row[b] = (((d0 * d0 + d1 * d1) + d2 * d2) + d3 * d3) + d4 * d4;
+            }
+        }
+    });
 
+    // The reference compares distances with the lower quartile of all of them.  The square root never reverses an order,
+    // so the quartile is the root of the quartile of the squares, and a distance lies below it exactly when its square
+    // lies below the smallest number whose root is the threshold.  Once everything is in one set, no pair changes
+    // anything any more.
+    cluster_parallel(cats.size(), pairs, [&](size_t i) {
+        Category& c = cats[i];
+        DisjointSet ds(c.m);
+        if (!c.squared.empty()) {
+            for (double x : c.squared) c.usable = c.usable && x == x;
+            double below;  // distances whose squares are below this
+            if (c.usable) {
+                below = cluster_select(c.squared, c.squared.size() / 4);
+                const double threshold = std::sqrt(below);
+                for (double d; below > 0 && std::sqrt(d = std::nextafter(below, 0.0)) == threshold;) below = d;
+            } else {  // not a number among the fingerprints: the order is what the library's selection makes of it
+                std::vector<double> sorted = c.squared;
+                for (double& x : sorted) x = std::sqrt(x);
+                std::nth_element(sorted.begin(), sorted.begin() + sorted.size() / 4, sorted.end());
+                const double threshold = sorted[sorted.size() / 4];
+                for (double& x : c.squared) x = std::sqrt(x);
+                below = threshold;
+            }
+            const double* p = c.squared.data();
+            int sets = c.m;
+            for (int a = 0; a < c.m && sets > 1; ++a)
+                for (int b = a + 1; b < c.m; ++b, ++p)
+                    if (*p < below) sets -= ds.unite(a, b);
+        }
+        c.root.resize(c.m);
+        for (int a = 0; a < c.m; ++a) c.root[a] = ds.find(a);
+    });
+
+    out.tensor_to_cluster.reserve(n);
+    for (const Category& c : cats) {
+        const std::vector<size_t>& idx = *c.idx;
+        const int m = c.m;
         std::map<int, std::vector<int>> by_root;
-        for (int a = 0; a < m; ++a) by_root[ds.find(a)].push_back(a);
+        for (int a = 0; a < m; ++a) by_root[c.root[a]].push_back(a);
         for (const auto& g : by_root) {
             const std::vector<int>& members = g.second;
             if (members.size() >= 2) {

@@ -4,6 +4,7 @@
 #include "cuda_emu.hpp"
 //
 #include "kernels.cuh"
+#include "clusters.hpp"
 #include "tables.hpp"
 
 #include <vector>
@@ -115,6 +116,26 @@ void emu_decode_split(size_t n, uint32_t planes, uint8_t* const* dsts, const uin
         emu::launch(grid, SplitSmem<1>::kChains + kSplitHelpers, sizeof(SplitSmem<1>), [&] { rans_decode_split_kernel<1>(fp); });
     else
         emu::launch(grid, SplitSmem<2>::kChains + kSplitHelpers, sizeof(SplitSmem<2>), [&] { rans_decode_split_kernel<2>(fp); });
+}
+
+// stats_slices1/2_kernel; outs: n * sizeof(StatsOut) bytes.
+void emu_stats_slices(size_t n, const void* const* ptrs, const uint64_t* n_elem, const uint32_t* dtype, uint32_t bins, void* outs) {
+    std::vector<StatsDesc> d(n);
+    for (size_t i = 0; i < n; ++i) d[i] = StatsDesc{ptrs[i], n_elem[i], dtype[i], bins};
+    std::memset(outs, 0, n * sizeof(StatsOut));
+    std::vector<float> p1(n * 768, -7.0f), p2(n * 768, -7.0f);
+    std::vector<uint32_t> done(n, 0);
+    SliceParams sp{d.data(), (StatsOut*)outs, p1.data(), p2.data(), done.data(), (uint32_t)n};
+    emu::launch((unsigned)n * kSlices, 32, 0, [&] { stats_slices1_kernel(sp); });
+    emu::launch((unsigned)n * kSlices, 32, 0, [&] { stats_slices2_kernel(sp); });
+}
+
+// build_clusters: cluster id per tensor (-1: none); returns the number of clusters.
+int emu_clusters(size_t n, const char* const* names, const float* fps, int32_t* ids) {
+    const std::vector<std::string> nm(names, names + n);
+    const ClusterMap m = build_clusters(nm, std::vector<float>(fps, fps + n * 5));
+    for (size_t i = 0; i < n; ++i) ids[i] = m.tensor_to_cluster.at(nm[i]);
+    return m.n_clusters;
 }
 
 }  // extern "C"

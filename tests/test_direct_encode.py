@@ -22,7 +22,7 @@ def direct_lib():
     srcs = [os.path.join(EMU_DIR, f) for f in ("emu_direct.cpp", "cuda_emu.hpp")] + \
            [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
     if not os.path.exists(so) or any(os.path.getmtime(so) < os.path.getmtime(s) for s in srcs):
-        subprocess.check_call(["g++", "-std=c++17", "-O1", "-I", CSRC, "-I", EMU_DIR, "-shared", "-fPIC", "-w", srcs[0], "-o", so])
+        subprocess.check_call(["g++", "-std=c++17", "-O1", "-pthread", "-I", CSRC, "-I", EMU_DIR, "-shared", "-fPIC", "-w", srcs[0], "-o", so])
     return C.CDLL(so)
 
 
@@ -211,6 +211,50 @@ def test_split_decode_of_planes(direct_lib, oracle, kind, es, misalign):
     assert not status.any()
     for d, w in zip(dsts, want):
         assert np.array_equal(d, w)
+
+
+@pytest.mark.parametrize("bins", [256, 64])
+def test_sliced_statistics_keep_the_reference_order(direct_lib, oracle, bins):
+    """Eight one-warp blocks per tensor, bit for bit: lengths around the 256 chains and the batches of loads."""
+    kinds = [("bf16_weight", 20000), ("f32_master", 4096), ("f32_master", 8192), ("f32_master", 8193), ("f32_master", 12288 + 255),
+             ("f32_exp_avg_sq_lognormal", 3 * 8192 + 77), ("f16_weight", 16384 + 255), ("i8", 300), ("i32", 1000),
+             ("f32_exp_avg_sq", 256), ("f32_master", 1), ("bf16_norm_gain", 513)]
+    tensors = batch(kinds, [1, 0, 2])
+    n = len(tensors)
+    ptrs = (C.c_void_p * n)(*[a.ctypes.data for a, _ in tensors])
+    ne = np.array([a.size // ELEM_SIZE[dt] for a, dt in tensors], np.uint64)
+    dts = np.array([dt for _, dt in tensors], np.uint32)
+    out = np.zeros((n, 268), np.uint32)
+    direct_lib.emu_stats_slices(C.c_size_t(n), ptrs, ne.ctypes.data_as(u64p), dts.ctypes.data_as(u32p), C.c_uint32(bins),
+                                out.ctypes.data_as(C.c_void_p))
+    for i, (a, dt) in enumerate(tensors):
+        h, mom, mm = oracle.tensor_stats(a, dt, bins)
+        assert np.array_equal(out[i, :256], h), kinds[i]
+        assert np.array_equal(out[i, 256:260], mom.view(np.uint32)), kinds[i]
+        assert np.array_equal(out[i, 260:262], mm.view(np.uint32)), kinds[i]
+
+
+@pytest.mark.parametrize("n,kind", [(1, "spread"), (2, "spread"), (3, "equal"), (60, "ties"), (200, "spread"), (400, "ties"),
+                                    (900, "groups"), (900, "spread"), (30, "nan")])
+def test_clusters_as_the_oracle_forms_them(direct_lib, oracle, n, kind):
+    """One and four categories, enough pairs for several threads, equal distances at the quartile."""
+    rng = np.random.default_rng(n)
+    fps = rng.normal(size=(n, 5)).astype(np.float32)
+    if kind == "equal":
+        fps[:] = 1.5
+    elif kind == "ties":
+        fps = rng.integers(0, 3, (n, 5)).astype(np.float32)
+    elif kind == "groups":
+        fps = (rng.integers(0, 40, (n, 1)) * 10 + fps * 0.01).astype(np.float32)
+    elif kind == "nan":
+        fps[7, 2] = np.nan
+    for prefixes in ([""], ["", "master_weights::", "optimizer.exp_avg::", "optimizer.exp_avg_sq::"]):
+        names = [prefixes[i % len(prefixes)] + f"t{i}" for i in range(n)]
+        ids = np.zeros(n, np.int32)
+        arr = (C.c_char_p * n)(*[s.encode() for s in names])
+        k = direct_lib.emu_clusters(C.c_size_t(n), arr, fps.ctypes.data_as(C.POINTER(C.c_float)), ids.ctypes.data_as(C.POINTER(C.c_int32)))
+        want, anchors = oracle.build_clusters(names, fps)
+        assert k == len(anchors) and np.array_equal(ids, want)
 
 
 @pytest.mark.gpu
