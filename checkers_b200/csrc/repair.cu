@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -70,36 +71,50 @@ struct PairKeyHash {  // same mixing as the reference's PairKeyHash (:363-371)
 // Device working set of one call.  One instance per device is kept for the life of the process and
 // only grows, so a run over many tensors does not pay an allocation per tensor.
 struct Workspace {
-    uint32_t n_cap = 0, capacity = 0;
+    uint32_t n_cap = 0, contiguous_cap = 0, capacity = 0;
     size_t raw_cap = 0;
-    bool ready = false;
     Dev tok_a, tok_b, mark, run_start, keep, pos, blocks, keys, counts, first, small, tie_keys, tie_first, dump_keys,
-        dump_counts, dump_first, raw;
+        dump_counts, dump_first, raw, tile_tok, tile_ends, tile_table, rules;
+    uint32_t rules_cap = 0;
+    bool smem_set = false;
     cudaStream_t s = nullptr;
+    std::mutex mu;          // one call at a time works on a device's workspace
     ~Workspace() {
         if (s) cudaStreamDestroy(s);
     }
-    void release() {
-        Dev* all[] = {&tok_a, &tok_b, &mark, &run_start, &keep, &pos, &blocks, &keys, &counts, &first, &small, &tie_keys,
-                      &tie_first, &dump_keys, &dump_counts, &dump_first, &raw};
+    static void drop(std::initializer_list<Dev*> all) {
         for (Dev* d : all) {
             if (d->p) cudaFree(d->p);
             d->p = nullptr;
         }
     }
+    // the tensor itself, its tiles and what goes with them
     void init(uint32_t n, size_t raw_bytes) {
-        if (ready && n <= n_cap && raw_bytes <= raw_cap) {
-            capacity = 1024;  // table sized for THIS tensor: the hash mask must match what is cleared
-            while (capacity < 2ull * n) capacity <<= 1;
-            return;
-        }
-        release();
-        n_cap = n;
-        raw_cap = raw_bytes;
-        capacity = 1024;
-        while (capacity < 2ull * n) capacity <<= 1;
         if (!s) RP_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        ready = true;
+        if (raw_bytes > raw_cap || !raw.p) {
+            drop({&raw});
+            raw_cap = 0;
+            raw.alloc(raw_bytes);
+            raw_cap = raw_bytes;
+        }
+        if (n > n_cap || !tile_tok.p) {
+            drop({&tile_tok, &tile_ends});
+            n_cap = 0;
+            const size_t tiles = ((size_t)n + kTile - 1) / kTile + 1;
+            tile_tok.alloc(2 * tiles * kTile * 2);
+            tile_ends.alloc(2 * tiles * sizeof(TileEnds));
+            n_cap = n;
+        }
+        if (!tile_table.p) tile_table.alloc(kTileTableBytes);
+    }
+    // what the kernels on contiguous sequences need
+    void init_contiguous(uint32_t n) {
+        capacity = 1024;  // table sized for THIS tensor: the hash mask must match what is cleared
+        while (capacity < 2ull * n) capacity <<= 1;
+        if (n <= contiguous_cap && tok_a.p) return;
+        drop({&tok_a, &tok_b, &mark, &run_start, &keep, &pos, &blocks, &keys, &counts, &first, &small, &tie_keys, &tie_first,
+              &dump_keys, &dump_counts, &dump_first});
+        contiguous_cap = 0;
         const size_t nb = (size_t)(n ? n : 1) * 4;
         tok_a.alloc(nb);
         tok_b.alloc(nb);
@@ -114,9 +129,20 @@ struct Workspace {
         small.alloc(64);
         tie_keys.alloc(64);
         tie_first.alloc(32);
-        raw.alloc(raw_bytes);
+        contiguous_cap = n;
     }
+    void ensure_rules(uint32_t n) {
+        if (n <= rules_cap) return;
+        drop({&rules});
+        rules_cap = 0;
+        rules.alloc((size_t)(n + 64) * 12);
+        rules_cap = n + 64;
+    }
+    // state, words that occur, numbers, words by number, matrix, two dumps
+    static constexpr size_t kMatrixBytes = (size_t)kDense * kDense * 4;
+    static constexpr size_t kTileTableBytes = 128 + 2 * (1u << kTileBits) + 512 + 3 * kMatrixBytes;
 };
+static_assert(sizeof(RoundState) <= 128 && kDense * 2 <= 512, "layout of the tile table");
 
 template <int OP>
 static void scan(Workspace& w, const uint32_t* in, uint32_t n, uint32_t* out) {
@@ -153,17 +179,193 @@ static uint32_t apply_rule(Workspace& w, const uint32_t* in, uint32_t n, uint32_
     return total;
 }
 
-static void upload_tokens(Workspace& w, const void* h_raw, uint64_t numel, uint32_t storage_bytes, uint32_t masked_bits) {
+// The tensor to the device.  (Filling a pinned buffer with several threads instead: 203 against 253 us for 4 MB, slower
+// below 2 MB, the same from 16 MB on.)
+static void upload_raw(Workspace& w, const void* h_raw, size_t bytes) {
+    if (bytes) RP_CUDA(cudaMemcpyAsync(w.raw.p, h_raw, bytes, cudaMemcpyHostToDevice, w.s));
+}
+
+static void mask_tokens(Workspace& w, uint64_t numel, uint32_t storage_bytes, uint32_t masked_bits) {
     if (numel == 0) return;
-    RP_CUDA(cudaMemcpyAsync(w.raw.p, h_raw, numel * storage_bytes, cudaMemcpyHostToDevice, w.s));
     mask_words_kernel<<<grid_for((uint32_t)numel), 256, 0, w.s>>>(w.raw.as<uint8_t>(), numel, storage_bytes, masked_bits,
                                                                   w.tok_a.as<uint32_t>());
     RP_CUDA(cudaGetLastError());
 }
 
+// ---- the tile path
+static TileParams tile_params(Workspace& w, uint32_t n, uint32_t max_rules) {
+    w.ensure_rules(max_rules + 1);
+    TileParams P{};
+    P.n_tiles = (n + kTile - 1) / kTile;
+    P.max_rules = max_rules;
+    P.tokens[0] = w.tile_tok.as<uint16_t>();
+    P.tokens[1] = P.tokens[0] + (size_t)P.n_tiles * kTile;
+    P.ends[0] = w.tile_ends.as<TileEnds>();
+    P.ends[1] = P.ends[0] + P.n_tiles;
+    P.rules = w.rules.as<uint2>();
+    P.rule_freq = reinterpret_cast<uint32_t*>(P.rules + w.rules_cap);
+    uint8_t* t = w.tile_table.as<uint8_t>();
+    P.state = reinterpret_cast<RoundState*>(t);
+    P.present = t + 128;
+    P.pairs = reinterpret_cast<uint32_t*>(P.present + (1u << kTileBits));
+    P.dump_counts = P.pairs + kDense * kDense;
+    P.dump_first = P.dump_counts + kDense * kDense;
+    P.number = reinterpret_cast<uint8_t*>(P.dump_first + kDense * kDense);
+    P.word_of = reinterpret_cast<uint16_t*>(P.number + (1u << kTileBits));
+    if (!w.smem_set) {  // per device
+        const int most = (int)tile_count_smem(kDense);
+        RP_CUDA(cudaFuncSetAttribute(tile_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        RP_CUDA(cudaFuncSetAttribute(tile_rule_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        RP_CUDA(cudaFuncSetAttribute(tile_dump_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most + (int)Workspace::kMatrixBytes));
+        w.smem_set = true;
+    }
+    return P;
+}
+
+// A launch that may begin while the one before it is still running (its kernel waits for that one itself).
+template <typename K, typename... A>
+static void launch_overlapping(cudaStream_t s, K kernel, uint32_t grid, size_t smem, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kTileThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    RP_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
+// token of the tiles <-> token id of the interface
+static uint32_t id_of_token(uint32_t t) { return t < kRuleToken ? t : kRuleBase + (t - kRuleToken); }
+static bool token_of_id(uint32_t id, uint32_t* t) {
+    if (id < kRuleToken) {
+        *t = id;
+        return true;
+    }
+    *t = kRuleToken + (id - kRuleBase);
+    return id >= kRuleBase && id - kRuleBase < kRuleToken;
+}
+
+// Which of several pairs with the largest count the reference's map yields first: the distinct pairs inserted in order of
+// their first position into a map built exactly like the reference's, and the map walked the same way.
+static unsigned long long first_in_map_order(const std::vector<unsigned long long>& hk, const std::vector<uint32_t>& hc,
+                                             const std::vector<uint32_t>& hf, uint32_t n_tokens, uint32_t masked_bits) {
+    const uint32_t d = (uint32_t)hk.size();
+    std::vector<uint32_t> order(d);
+    for (uint32_t i = 0; i < d; ++i) order[i] = i;
+    std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return hf[a] < hf[b]; });
+    std::unordered_map<PairKey, size_t, PairKeyHash> counts;
+    counts.reserve(n_tokens);
+    std::unordered_map<PairKey, unsigned long long, PairKeyHash> back;  // symbol pair -> id key
+    back.reserve(d);
+    for (uint32_t i : order) {
+        const PairKey pk{symbol_of((uint32_t)(hk[i] >> 32), masked_bits), symbol_of((uint32_t)hk[i], masked_bits)};
+        counts[pk] = hc[i];
+        back[pk] = hk[i];
+    }
+    size_t best_count = 0;
+    PairKey best_pair{};
+    for (const auto& kv : counts)
+        if (kv.second > best_count) {
+            best_count = kv.second;
+            best_pair = kv.first;
+        }
+    return back[best_pair];
+}
+
+// The grammar of the tensor in w.raw on tiles.  False: too many symbols, nothing has been decided.
+static bool build_on_tiles(Workspace& w, uint32_t numel, uint32_t storage_bytes, uint32_t masked_bits, uint32_t max_rules,
+                           uint32_t* rule_lhs, uint32_t* rule_rhs, uint64_t* rule_freq, uint32_t* n_rules_out,
+                           uint64_t* tokens_out, uint64_t* max_freq_out, uint64_t* tie_rounds_out) {
+    const TileParams P = tile_params(w, numel, max_rules);
+    RP_CUDA(cudaMemsetAsync(P.state, 0, 128 + (1u << kTileBits) + Workspace::kMatrixBytes, w.s));  // state, words, matrix
+    tile_words_kernel<true><<<P.n_tiles, kTileThreads, sizeof(TileCountSmem), w.s>>>(w.raw.as<uint8_t>(), numel, storage_bytes,
+                                                                                     masked_bits, P);
+    tile_pairs_kernel<<<P.n_tiles, kTileThreads, tile_count_smem(kDense), w.s>>>(P);
+    RP_CUDA(cudaGetLastError());
+    RoundState st{};
+    auto read_state = [&] {
+        RP_CUDA(cudaMemcpyAsync(&st, P.state, sizeof(st), cudaMemcpyDeviceToHost, w.s));
+        RP_CUDA(cudaStreamSynchronize(w.s));
+    };
+    read_state();
+    if (st.stop == kTooMany) return false;
+    uint64_t ties = 0;
+    uint32_t applied = 0;  // rules whose launch is queued
+    for (;;) {
+        if (st.stop == kNoMore) break;
+        if (st.stop == kTie) {
+            ++ties;
+            const uint32_t cells = st.side * st.side, current = st.n_rules - 1;
+            RP_CUDA(cudaMemsetAsync(P.dump_counts, 0, (size_t)cells * 4, w.s));
+            RP_CUDA(cudaMemsetAsync(P.dump_first, 0xFF, (size_t)cells * 4, w.s));
+            tile_dump_kernel<<<P.n_tiles, kTileThreads, tile_count_smem(st.side) + cells * 4, w.s>>>(P, current & 1u);
+            RP_CUDA(cudaGetLastError());
+            std::vector<uint32_t> counts(cells), first(cells);
+            std::vector<uint16_t> words(st.n_symbols);
+            RP_CUDA(cudaMemcpyAsync(counts.data(), P.dump_counts, (size_t)cells * 4, cudaMemcpyDeviceToHost, w.s));
+            RP_CUDA(cudaMemcpyAsync(first.data(), P.dump_first, (size_t)cells * 4, cudaMemcpyDeviceToHost, w.s));
+            RP_CUDA(cudaMemcpyAsync(words.data(), P.word_of, words.size() * 2, cudaMemcpyDeviceToHost, w.s));
+            RP_CUDA(cudaStreamSynchronize(w.s));
+            auto id = [&](uint32_t k) { return k < st.n_symbols ? (uint32_t)words[k] : kRuleBase + (k - st.n_symbols); };
+            std::vector<unsigned long long> hk;
+            std::vector<uint32_t> hc, hf;
+            for (uint32_t i = 0; i < cells; ++i)
+                if (counts[i]) {
+                    hk.push_back(((unsigned long long)id(i / st.side) << 32) | id(i % st.side));
+                    hc.push_back(counts[i]);
+                    hf.push_back(first[i]);
+                }
+            const unsigned long long key = first_in_map_order(hk, hc, hf, st.n_tokens, masked_bits);
+            uint2 rule;
+            token_of_id((uint32_t)(key >> 32), &rule.x);
+            token_of_id((uint32_t)key, &rule.y);
+            RP_CUDA(cudaMemcpyAsync(P.rules + current, &rule, sizeof(rule), cudaMemcpyHostToDevice, w.s));
+            const uint32_t go_on = kGoOn;
+            RP_CUDA(cudaMemcpyAsync(&P.state->stop, &go_on, 4, cudaMemcpyHostToDevice, w.s));
+            RP_CUDA(cudaStreamSynchronize(w.s));  // rule and go_on are on this stack frame
+            applied = current;
+        } else if (applied == max_rules) {
+            break;
+        }
+        // everything that may follow is queued at once; launches behind a stop do nothing.  Where one tie has come more
+        // are likely, so then a few at a time.
+        for (const uint32_t until = ties ? std::min(max_rules, applied + 8) : max_rules; applied < until; ++applied)
+            if (applied + 1 < max_rules)
+                launch_overlapping(w.s, tile_rule_kernel<true>, P.n_tiles, tile_count_smem(st.side), P, applied);
+            else
+                launch_overlapping(w.s, tile_rule_kernel<false>, P.n_tiles, sizeof(TileCountSmem), P, applied);
+        if (applied == max_rules) launch_overlapping(w.s, tile_total_kernel, 1, 0, P, max_rules & 1u);
+        read_state();
+    }
+    const uint32_t n_rules = st.n_rules;
+    std::vector<uint2> rules(n_rules);
+    std::vector<uint32_t> freq(n_rules);
+    if (n_rules) {
+        RP_CUDA(cudaMemcpyAsync(rules.data(), P.rules, (size_t)n_rules * 8, cudaMemcpyDeviceToHost, w.s));
+        RP_CUDA(cudaMemcpyAsync(freq.data(), P.rule_freq, (size_t)n_rules * 4, cudaMemcpyDeviceToHost, w.s));
+        RP_CUDA(cudaStreamSynchronize(w.s));
+    }
+    for (uint32_t r = 0; r < n_rules; ++r) {
+        if (rule_lhs) rule_lhs[r] = id_of_token(rules[r].x);
+        if (rule_rhs) rule_rhs[r] = id_of_token(rules[r].y);
+        if (rule_freq) rule_freq[r] = freq[r];
+    }
+    *n_rules_out = n_rules;
+    *tokens_out = st.n_tokens;
+    if (max_freq_out) *max_freq_out = st.max_freq;
+    if (tie_rounds_out) *tie_rounds_out = ties;
+    return true;
+}
+
 static Workspace& workspace_for(int device) {
     static Workspace* per_device[64] = {};
+    static std::mutex mu;
     if (device < 0 || device >= 64) throw Error{CHK_ERR_INVALID, "device ordinal out of range"};
+    std::lock_guard<std::mutex> lock(mu);
     if (!per_device[device]) per_device[device] = new Workspace();
     return *per_device[device];
 }
@@ -207,8 +409,15 @@ int chk_repair_build(int device, const void* h_raw, uint64_t numel, uint32_t sto
     check_args(numel, storage_bytes, masked_bits);
     RP_CUDA(cudaSetDevice(device));
     Workspace& w = workspace_for(device);
+    std::lock_guard<std::mutex> lock(w.mu);
     w.init((uint32_t)numel, numel * storage_bytes);
-    upload_tokens(w, h_raw, numel, storage_bytes, masked_bits);
+    upload_raw(w, h_raw, numel * storage_bytes);
+    if (numel && max_rules && max_rules < kDense && storage_bytes * 8 - masked_bits <= kTileBits &&
+        build_on_tiles(w, (uint32_t)numel, storage_bytes, masked_bits, max_rules, rule_lhs, rule_rhs, rule_freq, n_rules_out,
+                       tokens_out, max_pair_frequency_out, tie_rounds_out))
+        return CHK_OK;
+    w.init_contiguous((uint32_t)numel);
+    mask_tokens(w, numel, storage_bytes, masked_bits);
     uint32_t* cur = w.tok_a.as<uint32_t>();
     uint32_t* nxt = w.tok_b.as<uint32_t>();
     uint32_t n = (uint32_t)numel, n_rules = 0;
@@ -242,9 +451,9 @@ int chk_repair_build(int device, const void* h_raw, uint64_t numel, uint32_t sto
             // several pairs share the maximum: replay the reference's map to see which it meets first
             ++tie_rounds;
             if (!w.dump_keys.p) {
-                w.dump_keys.alloc((size_t)w.n_cap * 8 + 8);
-                w.dump_counts.alloc((size_t)w.n_cap * 4 + 4);
-                w.dump_first.alloc((size_t)w.n_cap * 4 + 4);
+                w.dump_keys.alloc((size_t)w.contiguous_cap * 8 + 8);
+                w.dump_counts.alloc((size_t)w.contiguous_cap * 4 + 4);
+                w.dump_first.alloc((size_t)w.contiguous_cap * 4 + 4);
             }
             pair_dump_kernel<<<grid_for(w.capacity), 256, 0, w.s>>>(
                 w.keys.as<unsigned long long>(), w.counts.as<uint32_t>(), w.first.as<uint32_t>(), w.capacity, small + 3,
@@ -258,26 +467,7 @@ int chk_repair_build(int device, const void* h_raw, uint64_t numel, uint32_t sto
             RP_CUDA(cudaMemcpy(hk.data(), w.dump_keys.p, (size_t)d * 8, cudaMemcpyDeviceToHost));
             RP_CUDA(cudaMemcpy(hc.data(), w.dump_counts.p, (size_t)d * 4, cudaMemcpyDeviceToHost));
             RP_CUDA(cudaMemcpy(hf.data(), w.dump_first.p, (size_t)d * 4, cudaMemcpyDeviceToHost));
-            std::vector<uint32_t> order(d);
-            for (uint32_t i = 0; i < d; ++i) order[i] = i;
-            std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return hf[a] < hf[b]; });
-            std::unordered_map<PairKey, size_t, PairKeyHash> counts;
-            counts.reserve(n);
-            std::unordered_map<PairKey, unsigned long long, PairKeyHash> back;  // symbol pair -> id key
-            back.reserve(d);
-            for (uint32_t i : order) {
-                const PairKey pk{symbol_of((uint32_t)(hk[i] >> 32), masked_bits), symbol_of((uint32_t)hk[i], masked_bits)};
-                counts[pk] = hc[i];
-                back[pk] = hk[i];
-            }
-            size_t best_count = 0;
-            PairKey best_pair{};
-            for (const auto& kv : counts)
-                if (kv.second > best_count) {
-                    best_count = kv.second;
-                    best_pair = kv.first;
-                }
-            key = back[best_pair];
+            key = first_in_map_order(hk, hc, hf, n, masked_bits);
         }
         const uint32_t lhs = (uint32_t)(key >> 32), rhs = (uint32_t)key, sym = kRuleBase + n_rules;
         const uint32_t m = apply_rule(w, cur, n, lhs, rhs, sym, nxt);
@@ -304,16 +494,41 @@ int chk_repair_apply(int device, const void* h_raw, uint64_t numel, uint32_t sto
     check_args(numel, storage_bytes, masked_bits);
     RP_CUDA(cudaSetDevice(device));
     Workspace& w = workspace_for(device);
-    w.init((uint32_t)numel, numel * storage_bytes);
-    upload_tokens(w, h_raw, numel, storage_bytes, masked_bits);
-    uint32_t* cur = w.tok_a.as<uint32_t>();
-    uint32_t* nxt = w.tok_b.as<uint32_t>();
+    std::lock_guard<std::mutex> lock(w.mu);
     uint32_t n = (uint32_t)numel;
-    for (uint32_t r = 0; r < n_rules; ++r) {
-        n = apply_rule(w, cur, n, rule_lhs[r], rule_rhs[r], kRuleBase + r, nxt);
-        std::swap(cur, nxt);
+    if (!n || !n_rules) {
+        *tokens_out = n;
+        return CHK_OK;
     }
-    RP_CUDA(cudaStreamSynchronize(w.s));
+    w.init(n, numel * storage_bytes);
+    upload_raw(w, h_raw, numel * storage_bytes);
+    std::vector<uint2> rules(n_rules);
+    bool on_tiles = storage_bytes * 8 - masked_bits <= 15 && n_rules < kRuleToken;  // 16-bit tokens
+    for (uint32_t r = 0; r < n_rules && on_tiles; ++r)
+        on_tiles = token_of_id(rule_lhs[r], &rules[r].x) && token_of_id(rule_rhs[r], &rules[r].y);
+    if (on_tiles) {
+        const TileParams P = tile_params(w, n, n_rules);
+        RP_CUDA(cudaMemcpyAsync(P.rules, rules.data(), (size_t)n_rules * 8, cudaMemcpyHostToDevice, w.s));
+        RP_CUDA(cudaMemsetAsync(P.state, 0, sizeof(RoundState), w.s));
+        tile_words_kernel<false><<<P.n_tiles, kTileThreads, sizeof(TileCountSmem), w.s>>>(w.raw.as<uint8_t>(), numel, storage_bytes,
+                                                                                          masked_bits, P);
+        for (uint32_t r = 0; r < n_rules; ++r)
+            launch_overlapping(w.s, tile_rule_kernel<false>, P.n_tiles, sizeof(TileCountSmem), P, r);
+        launch_overlapping(w.s, tile_total_kernel, 1, 0, P, n_rules & 1u);
+        RoundState st{};
+        RP_CUDA(cudaMemcpyAsync(&st, P.state, sizeof(st), cudaMemcpyDeviceToHost, w.s));
+        RP_CUDA(cudaStreamSynchronize(w.s));
+        n = st.n_tokens;
+    } else {
+        w.init_contiguous(n);
+        mask_tokens(w, numel, storage_bytes, masked_bits);
+        uint32_t* cur = w.tok_a.as<uint32_t>();
+        uint32_t* nxt = w.tok_b.as<uint32_t>();
+        for (uint32_t r = 0; r < n_rules; ++r) {
+            n = apply_rule(w, cur, n, rule_lhs[r], rule_rhs[r], kRuleBase + r, nxt);
+            std::swap(cur, nxt);
+        }
+    }
     *tokens_out = n;
     RP_END
 }

@@ -15,6 +15,7 @@
 //                       data-parallel stream compaction (a run of equal symbols
 //                       under a rule (a,a) is paired from its start, as the
 //                       sequential scan does)
+//   tile_*_kernel       the same on tiles, for sequences of few symbols and for applying a finished grammar
 // Included by repair.cu and by the CPU emulator build of the test suite.
 #pragma once
 #include <stdint.h>
@@ -27,8 +28,12 @@ constexpr uint32_t kScanBlock = 1024;        // elements per block in the scan p
 
 #ifdef CHK_CPU_EMULATION
 #define CHKRP_SHARED static
+#define CHKRP_DYN_SMEM(p) unsigned char* p = (unsigned char*)(((uintptr_t)emu::g_dyn_smem.data() + 127) & ~(uintptr_t)127)
 #else
 #define CHKRP_SHARED __shared__
+#define CHKRP_DYN_SMEM(p)                                             \
+    extern __shared__ __align__(128) unsigned char chkrp_dyn_smem_[]; \
+    unsigned char* p = chkrp_dyn_smem_
 #endif
 
 // words: little-endian storage of the tensor (2 or 4 bytes per element) -> token ids
@@ -272,6 +277,498 @@ __global__ void __launch_bounds__(256) rule_scatter_kernel(const uint32_t* __res
                                                            uint32_t* __restrict__ out) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         if (keep[i]) out[pos[i]] = pair_taken(tokens, n, i, lhs, rhs, run_start) ? new_sym : tokens[i];
+}
+
+// ---- few symbols: tiles and a dense pair matrix, nothing for the host to wait for between rules ----
+// With the mantissa masked a tensor has a few dozen distinct words.  Such a sequence is held as tiles of up to kTile
+// 16-bit tokens (the word, or 0x8000 + r for rule r), each shrinking in a place of its own, so a rewrite needs no scan over
+// the sequence: one block per tile, one launch per rule.  What crosses a tile's border follows from what every tile
+// says about its ends.
+//   Counts.  The pairs inside tiles are counted once, into a matrix over the symbols present and the rules to come.
+// A rule then changes only the pairs that touch a replaced one: a tile takes those off and adds the ones around the new
+// symbol, first in a matrix in shared memory, then -- the entries that changed -- in the global one.  The block that
+// finishes a launch last (a counter; nobody waits) adds the pairs across borders to its copy of the matrix and picks
+// the next rule, so all launches are queued at once.  When several pairs share the maximum the launches behind do
+// nothing until the host has chosen (tile_dump_kernel brings it the pairs).
+//   Sequences with more symbols than the matrix has room for are left to the kernels above.  A round over 2^20 tokens
+// takes 18 us (7 without counting); through the kernels above, with two waits for the host, 110 (40).
+constexpr uint32_t kTile = 4096, kTileThreads = 512, kTilePer = kTile / kTileThreads;
+constexpr uint32_t kDense = 144;              // symbols and rules the matrix has room for
+constexpr uint32_t kTileBits = 12;            // width of a masked word that can be counted this way
+constexpr uint32_t kRuleToken = 0x8000u;
+
+struct alignas(16) TileEnds {     // of every tile
+    uint32_t len, first, last;
+    uint32_t trail;   // equal tokens at the end
+};
+enum : uint32_t { kGoOn = 0, kNoMore = 1, kTie = 2, kTooMany = 3 };
+struct RoundState {
+    uint32_t stop;        // kGoOn, or why the launches after this one do nothing
+    uint32_t n_rules;     // rules chosen so far
+    uint32_t n_tokens;
+    uint32_t best, ties;  // of the last count
+    uint32_t max_freq;
+    uint32_t n_symbols;   // distinct words
+    uint32_t side;        // of the matrix: n_symbols + the rules asked for, rounded up to a multiple of 4
+    uint32_t done;
+};
+struct TileParams {
+    uint32_t n_tiles;
+    uint32_t max_rules;
+    uint16_t* tokens[2];      // n_tiles * kTile each; rule r reads [r & 1] and writes the other
+    TileEnds* ends[2];
+    uint2* rules;             // {lhs, rhs}
+    uint32_t* rule_freq;      // how often the chosen pair was counted
+    RoundState* state;
+    uint8_t* present;         // [1 << kTileBits], zeroed: words that occur
+    uint8_t* number;          // [1 << kTileBits] word -> symbol number
+    uint16_t* word_of;        // [kDense] symbol number -> word
+    uint32_t* pairs;          // [kDense * kDense], zeroed: pairs inside tiles
+    uint32_t* dump_counts;    // on a tie: all pairs, zeroed,
+    uint32_t* dump_first;     // and where each is met first, all ones
+};
+
+struct TileSmem {
+    uint16_t in[kTile], out[kTile];
+    uint16_t first[kTileThreads + 1], last[kTileThreads + 1];  // every thread's end tokens
+    uint8_t touched[kTileThreads + 1];                         // whether its last token is part of a replaced pair
+    uint32_t part[kTileThreads / 32];
+    uint32_t prev, next, carry, last_other, is_last, stop_at;
+    uint32_t best, ties, total;
+};
+struct TileCountSmem {
+    TileSmem rule;
+    alignas(16) uint8_t number[1u << kTileBits];  // word -> symbol number
+    alignas(16) uint32_t pairs[4];                // side * side (as many as the launch provides)
+};
+inline uint32_t tile_count_smem(uint32_t side) { return (uint32_t)sizeof(TileCountSmem) + side * side * 4; }
+
+// What other blocks of this launch may have written is read past L1.
+#ifdef CHK_CPU_EMULATION
+__device__ __forceinline__ uint4 read_l2(const uint4* p) { return *p; }
+__device__ __forceinline__ uint32_t read_l2(const uint32_t* p) { return *p; }
+__device__ __forceinline__ void tile_launch_next() {}
+__device__ __forceinline__ void tile_wait_previous() {}
+#else
+__device__ __forceinline__ uint4 read_l2(const uint4* p) { return __ldcg(p); }
+__device__ __forceinline__ uint32_t read_l2(const uint32_t* p) { return __ldcg(p); }
+// Rule launches overlap: the next one may start as soon as every block has begun, and waits for this one's end (and its
+// writes) before it reads anything.
+__device__ __forceinline__ void tile_launch_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void tile_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+__device__ __forceinline__ TileEnds ends_at(const TileEnds* e, uint32_t t) {
+    const uint4 q = read_l2(reinterpret_cast<const uint4*>(e + t));
+    return TileEnds{q.x, q.y, q.z, q.w};
+}
+
+__device__ __forceinline__ uint32_t symbol_of_token(const TileCountSmem* cs, uint32_t n_symbols, uint32_t t) {
+    return t < kRuleToken ? (uint32_t)cs->number[t] : n_symbols + (t - kRuleToken);
+}
+// The first token behind tile t.
+__device__ __forceinline__ bool tile_next_first(const TileEnds* e, uint32_t n_tiles, uint32_t t, uint32_t* first) {
+    for (++t; t < n_tiles; ++t) {
+        const TileEnds q = ends_at(e, t);
+        if (q.len) {
+            *first = q.first;
+            return true;
+        }
+    }
+    return false;
+}
+
+// Exclusive sum over the block's threads.
+__device__ __forceinline__ uint32_t tile_scan(uint32_t v, uint32_t* part, uint32_t* total) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += n;
+    }
+    __syncthreads();
+    if (lane == 31) part[warp] = inc;
+    __syncthreads();
+    uint32_t before = 0, sum = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kTileThreads / 32; ++w) {
+        if (w < warp) before += part[w];
+        sum += part[w];
+    }
+    *total = sum;
+    return before + inc - v;
+}
+// Maximum over the threads before this one (0 for the first).
+__device__ __forceinline__ uint32_t tile_max_before(uint32_t v, uint32_t* part) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o && n > inc) inc = n;
+    }
+    __syncthreads();
+    if (lane == 31) part[warp] = inc;
+    __syncthreads();
+    uint32_t before = 0;
+    for (uint32_t w = 0; w < warp; ++w) before = part[w] > before ? part[w] : before;
+    const uint32_t left = __shfl_up_sync(0xffffffffu, inc, 1);
+    return lane && left > before ? left : before;
+}
+
+// The tile in sm->out[0..len) to memory, with what it says about its ends.
+__device__ __forceinline__ void tile_store(TileSmem* sm, uint32_t len, uint16_t* out, TileEnds* e) {
+    const uint32_t tid = threadIdx.x;
+    if (tid == 0) sm->last_other = 0;
+    __syncthreads();
+    const uint32_t last = len ? sm->out[len - 1] : 0u;
+    const uint4 q = reinterpret_cast<const uint4*>(sm->out)[tid];
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w}, lo = tid * kTilePer;
+    uint32_t other = 0;  // 1 + the last position of this thread's that holds another token
+#pragma unroll
+    for (uint32_t k = 0; k < kTilePer; ++k)
+        if (lo + k < len && ((w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu) != last) other = lo + k + 1;
+    if (other > *(volatile uint32_t*)&sm->last_other) atomicMax(&sm->last_other, other);
+    if (lo < len) *reinterpret_cast<uint4*>(out + lo) = q;
+    __syncthreads();
+    if (tid == 0) {
+        e->len = len;
+        e->first = len ? sm->out[0] : 0u;
+        e->last = last;
+        e->trail = len - sm->last_other;
+    }
+}
+
+// Word -> symbol number from the words that occur; returns how many there are.
+__device__ __forceinline__ uint32_t tile_number_words(const TileParams& P, TileCountSmem* cs) {
+    constexpr uint32_t kEach = (1u << kTileBits) / kTileThreads;
+    uint32_t mine = 0, total;
+    for (uint32_t k = 0; k < kEach; ++k) mine += P.present[threadIdx.x * kEach + k];
+    uint32_t at = tile_scan(mine, cs->rule.part, &total);
+    for (uint32_t k = 0; k < kEach; ++k) {
+        cs->number[threadIdx.x * kEach + k] = (uint8_t)at;
+        at += P.present[threadIdx.x * kEach + k];
+    }
+    __syncthreads();
+    return total;
+}
+
+__device__ __forceinline__ void tile_load_numbers(const TileParams& P, TileCountSmem* cs) {
+    static_assert((1u << kTileBits) == 8 * kTileThreads, "eight numbers a thread");
+    reinterpret_cast<uint2*>(cs->number)[threadIdx.x] = reinterpret_cast<const uint2*>(P.number)[threadIdx.x];
+}
+
+__device__ __forceinline__ void tile_clear(uint32_t* pairs, uint32_t n) {  // n: a multiple of 4
+    for (uint32_t i = threadIdx.x; i < n / 4; i += kTileThreads) reinterpret_cast<uint4*>(pairs)[i] = make_uint4(0, 0, 0, 0);
+}
+__device__ __forceinline__ void tile_add_to(uint32_t* all, const uint32_t* pairs, uint32_t n) {  // what is not zero
+    for (uint32_t i = threadIdx.x; i < n / 4; i += kTileThreads) {
+        const uint4 q = reinterpret_cast<const uint4*>(pairs)[i];
+        if (!(q.x | q.y | q.z | q.w)) continue;
+        if (q.x) atomicAdd(&all[4 * i], q.x);
+        if (q.y) atomicAdd(&all[4 * i + 1], q.y);
+        if (q.z) atomicAdd(&all[4 * i + 2], q.z);
+        if (q.w) atomicAdd(&all[4 * i + 3], q.w);
+    }
+}
+
+// The block that finishes last takes the pairs of all tiles together and picks the next rule.
+__device__ __forceinline__ void tile_choose(const TileParams& P, TileCountSmem* cs, const TileEnds* e, uint32_t rules_applied,
+                                            uint32_t n_symbols, uint32_t side) {
+    TileSmem* const sm = &cs->rule;
+    RoundState* const st = P.state;
+    const uint32_t tid = threadIdx.x;
+    const volatile uint16_t* const word_of = P.word_of;
+    const uint32_t used = (n_symbols + rules_applied) * side;  // rows of symbols and rules that occur
+#pragma unroll 4
+    for (uint32_t i = tid; i < used / 4; i += kTileThreads)
+        reinterpret_cast<uint4*>(cs->pairs)[i] = read_l2(reinterpret_cast<const uint4*>(P.pairs) + i);
+    if (tid == 0) sm->best = sm->ties = sm->total = 0;
+    __syncthreads();
+    uint32_t mine = 0;
+    for (uint32_t q = tid; q < P.n_tiles; q += kTileThreads) {
+        const TileEnds own = ends_at(e, q), next = ends_at(e, q + 1 < P.n_tiles ? q + 1 : q);
+        uint32_t nx = next.first;
+        mine += own.len;
+        if (own.len && q + 1 < P.n_tiles && (next.len || tile_next_first(e, P.n_tiles, q + 1, &nx)))
+            atomicAdd(&cs->pairs[symbol_of_token(cs, n_symbols, own.last) * side + symbol_of_token(cs, n_symbols, nx)], 1u);
+    }
+    if (mine) atomicAdd(&sm->total, mine);
+    __syncthreads();
+    uint32_t m = 0;
+    for (uint32_t i = tid; i < used / 4; i += kTileThreads) {
+        const uint4 q = reinterpret_cast<const uint4*>(cs->pairs)[i];
+        const uint32_t xy = q.x > q.y ? q.x : q.y, zw = q.z > q.w ? q.z : q.w, most = xy > zw ? xy : zw;
+        m = most > m ? most : m;
+    }
+    if (m > *(volatile uint32_t*)&sm->best) atomicMax(&sm->best, m);
+    __syncthreads();
+    const uint32_t best = sm->best;
+    // the thread's own largest tells it whether to look again
+    for (uint32_t i = m == best && best ? tid : used; i < used / 4; i += kTileThreads)
+        for (uint32_t c = 0; c < 4; ++c) {
+            if (cs->pairs[4 * i + c] != best) continue;
+            atomicAdd(&sm->ties, 1u);
+            const uint32_t l = (4 * i + c) / side, r = (4 * i + c) % side;  // the only pair, unless there is a tie
+            P.rules[rules_applied] = make_uint2(l < n_symbols ? (uint32_t)word_of[l] : kRuleToken + (l - n_symbols),
+                                                r < n_symbols ? (uint32_t)word_of[r] : kRuleToken + (r - n_symbols));
+        }
+    __syncthreads();
+    if (tid == 0) {
+        st->done = 0;
+        st->n_tokens = sm->total;
+        st->best = best;
+        st->ties = sm->ties;
+        if (best > st->max_freq) st->max_freq = best;
+        if (sm->total < 2 || best < 2) {
+            st->stop = kNoMore;
+        } else {
+            P.rule_freq[rules_applied] = best;
+            st->n_rules = rules_applied + 1;
+            if (sm->ties > 1) st->stop = kTie;
+        }
+    }
+}
+__device__ __forceinline__ bool tile_is_last(const TileParams& P, TileSmem* sm) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) sm->is_last = atomicAdd(&P.state->done, 1u) + 1u == P.n_tiles;
+    __syncthreads();
+    if (!sm->is_last) return false;
+    __threadfence();
+    return true;
+}
+
+// words of the tensor -> tokens in tiles; kMark: also which words occur
+template <bool kMark>
+__global__ void __launch_bounds__(kTileThreads) tile_words_kernel(const uint8_t* __restrict__ raw, unsigned long long n,
+                                                                  uint32_t storage_bytes, uint32_t masked_bits, const TileParams P) {
+    CHKRP_DYN_SMEM(smem);
+    TileCountSmem* const cs = reinterpret_cast<TileCountSmem*>(smem);
+    TileSmem* const sm = &cs->rule;
+    const uint32_t t = blockIdx.x, tid = threadIdx.x;
+    const unsigned long long base = (unsigned long long)t * kTile;
+    const uint32_t len = n - base < kTile ? (uint32_t)(n - base) : kTile;
+    if (kMark)
+        for (uint32_t i = tid; i < (1u << kTileBits); i += kTileThreads) cs->number[i] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < len; i += kTileThreads) {
+        const uint32_t w = (storage_bytes == 4 ? reinterpret_cast<const uint32_t*>(raw)[base + i]
+                                               : (uint32_t)reinterpret_cast<const uint16_t*>(raw)[base + i]) >> masked_bits;
+        sm->out[i] = (uint16_t)w;
+        if (kMark) cs->number[w] = 1;
+    }
+    __syncthreads();
+    if (kMark)
+        for (uint32_t i = tid; i < (1u << kTileBits); i += kTileThreads)
+            if (cs->number[i]) P.present[i] = 1;
+    tile_store(sm, len, P.tokens[0] + base, &P.ends[0][t]);
+}
+
+// The pairs inside the tiles, and the first rule.
+__global__ void __launch_bounds__(kTileThreads) tile_pairs_kernel(const TileParams P) {
+    CHKRP_DYN_SMEM(smem);
+    TileCountSmem* const cs = reinterpret_cast<TileCountSmem*>(smem);
+    RoundState* const st = P.state;
+    const uint32_t t = blockIdx.x, tid = threadIdx.x;
+    const uint32_t n_symbols = tile_number_words(P, cs), side = (n_symbols + P.max_rules + 3u) & ~3u;
+    if (side > kDense) {  // the same for every block
+        if (tid == 0) st->stop = kTooMany;
+        return;
+    }
+    if (t == 0) {
+        for (uint32_t i = tid; i < (1u << kTileBits); i += kTileThreads) {
+            P.number[i] = cs->number[i];
+            if (P.present[i]) P.word_of[cs->number[i]] = (uint16_t)i;
+        }
+        if (tid == 0) {
+            st->n_symbols = n_symbols;
+            st->side = side;
+        }
+    }
+    tile_clear(cs->pairs, side * side);
+    __syncthreads();
+    const uint32_t len = P.ends[0][t].len;
+    const uint16_t* const in = P.tokens[0] + (size_t)t * kTile;
+    for (uint32_t i = tid; i + 1 < len; i += kTileThreads) atomicAdd(&cs->pairs[cs->number[in[i]] * side + cs->number[in[i + 1]]], 1u);
+    __syncthreads();
+    tile_add_to(P.pairs, cs->pairs, side * side);
+    if (tile_is_last(P, &cs->rule)) tile_choose(P, cs, P.ends[0], 0, n_symbols, side);
+}
+
+// Applies rule `rule`; kCount: and updates the counts and picks the next rule.
+template <bool kCount>
+__global__ void __launch_bounds__(kTileThreads) tile_rule_kernel(const TileParams P, uint32_t rule) {
+    CHKRP_DYN_SMEM(smem);
+    TileCountSmem* const cs = reinterpret_cast<TileCountSmem*>(smem);
+    TileSmem* const sm = &cs->rule;
+    RoundState* const st = P.state;
+    const uint32_t t = blockIdx.x, tid = threadIdx.x, from = rule & 1u;
+    const TileEnds* const e = from ? P.ends[1] : P.ends[0];  // (selected: indexing the parameter would copy it to local memory)
+    TileEnds* const e_out = from ? P.ends[0] : P.ends[1];
+    const uint16_t* const tokens_in = (from ? P.tokens[1] : P.tokens[0]) + (size_t)t * kTile;
+    uint16_t* const tokens_out = (from ? P.tokens[0] : P.tokens[1]) + (size_t)t * kTile;
+    const uint32_t lo = tid * kTilePer;
+    tile_launch_next();
+    tile_wait_previous();
+    // everything a block needs from memory is requested before the first of it is looked at
+    const uint32_t stop = read_l2(&st->stop);
+    const uint32_t a = read_l2(&P.rules[rule].x), b = read_l2(&P.rules[rule].y), sym = kRuleToken + rule;
+    const TileEnds own = ends_at(e, t), next_tile = ends_at(e, t + 1 < P.n_tiles ? t + 1 : t), prev_tile = ends_at(e, t ? t - 1 : 0u);
+    const uint4 q = read_l2(reinterpret_cast<const uint4*>(tokens_in + lo));
+    uint32_t side = 0, n_symbols = 0;
+    if (kCount) {
+        side = read_l2(&st->side);
+        n_symbols = read_l2(&st->n_symbols);
+    }
+    if (stop != kGoOn) return;
+    const uint32_t len = own.len, cnt = lo < len ? (len - lo < kTilePer ? len - lo : kTilePer) : 0u;
+    uint32_t v[kTilePer];
+    {
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (uint32_t k = 0; k < kTilePer; ++k) v[k] = (w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
+    }
+    if (kCount) {
+        tile_clear(cs->pairs, (n_symbols + rule + 1) * side);
+        tile_load_numbers(P, cs);
+        reinterpret_cast<uint4*>(sm->in)[tid] = q;
+    }
+    sm->first[tid] = (uint16_t)v[0];
+    sm->last[tid] = (uint16_t)v[kTilePer - 1];
+    if (tid == 0) {
+        uint32_t nx = next_tile.first;
+        sm->next = t + 1 < P.n_tiles && (next_tile.len || tile_next_first(e, P.n_tiles, t + 1, &nx)) && nx == b;  // the token after the tile completes a pair
+        TileEnds before = prev_tile;
+        for (uint32_t p = t; p > 1 && !before.len;) before = ends_at(e, --p - 1);
+        sm->prev = t && before.len && before.last == a;  // the token before it does
+        sm->carry = 0;
+        sm->stop_at = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    if (a == b) {
+        // equal tokens right before the tile: whole tiles of them, then the end of another
+        for (uint32_t base = 0; base < t; base += kTileThreads) {
+            const uint32_t q = base + tid;  // tile t - 1 - q
+            TileEnds pe{0, 0, 0, 0};
+            if (q < t) pe = ends_at(e, t - 1 - q);
+            if (q < t && pe.len && (pe.last != a || pe.trail < pe.len)) atomicMin(&sm->stop_at, q);
+            __syncthreads();
+            const uint32_t stop_at = sm->stop_at;
+            const uint32_t mine = q < t && q <= stop_at && pe.len && pe.last == a ? pe.trail : 0u;
+            if (mine) atomicAdd(&sm->carry, mine);
+            __syncthreads();
+            if (stop_at != 0xFFFFFFFFu) break;
+        }
+    }
+    const uint32_t before = tid ? sm->last[tid - 1] : 0u, after = tid + 1 < kTileThreads ? sm->first[tid + 1] : 0u;
+    uint32_t run = 0;  // (a, a): 1 + the last position before `lo` that holds another token
+    if (a == b) {
+        uint32_t other = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kTilePer; ++k)
+            if (k < cnt && v[k] != a) other = lo + k + 1;
+        run = tile_max_before(other, sm->part);
+    }
+    uint32_t second = 0, firsts = 0;  // masks of second and first halves of replaced pairs
+#pragma unroll
+    for (uint32_t k = 0; k < kTilePer; ++k) {
+        const uint32_t i = lo + k;
+        if (k >= cnt) continue;
+        const bool follows = i + 1 < len ? (k + 1 < kTilePer ? v[(k + 1) % kTilePer] : after) == b : sm->next != 0;
+        bool f, s;
+        if (a != b) {
+            f = v[k] == a && follows;
+            s = v[k] == b && (i ? (k ? v[(k + kTilePer - 1) % kTilePer] : before) == a : sm->prev != 0);
+        } else {  // pairs are formed from the start of the run
+            const uint32_t at = i - run + (run == 0 ? sm->carry : 0u);
+            f = v[k] == a && (at & 1u) == 0 && follows;
+            s = v[k] == a && (at & 1u) != 0;
+            if (v[k] != a) run = i + 1;
+        }
+        second |= s ? 1u << k : 0u;
+        firsts |= f ? 1u << k : 0u;
+    }
+    uint32_t new_len;
+    uint32_t at = tile_scan(cnt - (uint32_t)__popc(second), sm->part, &new_len);
+#pragma unroll
+    for (uint32_t k = 0; k < kTilePer; ++k)
+        if (k < cnt && !(second & (1u << k))) sm->out[at++] = (uint16_t)(firsts & (1u << k) ? sym : v[k]);
+    const uint32_t touched = second | firsts;
+    if (kCount) sm->touched[tid] = (uint8_t)((touched >> (kTilePer - 1)) & 1u);
+    __syncthreads();
+    if (kCount) {
+        // off with the pairs that touch a replaced one ...
+        uint32_t pairs = (touched | (touched << 1) | (tid ? sm->touched[tid - 1] : 0u)) & ((1u << cnt) - 1u);
+        for (pairs &= lo ? ~0u : ~1u; pairs; pairs &= pairs - 1) {
+            const uint32_t j = lo + (uint32_t)__ffs(pairs) - 1u;
+            atomicAdd(&cs->pairs[symbol_of_token(cs, n_symbols, sm->in[j - 1]) * side + symbol_of_token(cs, n_symbols, sm->in[j])],
+                      0xFFFFFFFFu);
+        }
+        // ... and on with those around the new symbol
+        const uint4 nq = reinterpret_cast<const uint4*>(sm->out)[tid];
+        const uint32_t w[4] = {nq.x, nq.y, nq.z, nq.w};
+        uint32_t fresh = lo && sm->out[lo - 1] == sym ? 1u : 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < kTilePer; ++k) fresh |= ((w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu) == sym ? 3u << k : 0u;
+        fresh &= (1u << (lo < new_len ? (new_len - lo < kTilePer ? new_len - lo : kTilePer) : 0u)) - 1u;
+        for (fresh &= lo ? ~0u : ~1u; fresh; fresh &= fresh - 1) {
+            const uint32_t j = lo + (uint32_t)__ffs(fresh) - 1u;
+            atomicAdd(&cs->pairs[symbol_of_token(cs, n_symbols, sm->out[j - 1]) * side + symbol_of_token(cs, n_symbols, sm->out[j])], 1u);
+        }
+        __syncthreads();
+        tile_add_to(P.pairs, cs->pairs, (n_symbols + rule + 1) * side);
+    }
+    tile_store(sm, new_len, tokens_out, &e_out[t]);
+    if (kCount && tile_is_last(P, sm)) tile_choose(P, cs, e_out, rule + 1, n_symbols, side);
+}
+
+// Tokens in all tiles of a buffer.
+__global__ void __launch_bounds__(kTileThreads) tile_total_kernel(const TileParams P, uint32_t buffer) {
+    CHKRP_SHARED uint32_t total;
+    tile_wait_previous();
+    if (P.state->stop != kGoOn) return;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    uint32_t mine = 0;
+    for (uint32_t q = threadIdx.x; q < P.n_tiles; q += kTileThreads) mine += (buffer ? P.ends[1] : P.ends[0])[q].len;
+    if (mine) atomicAdd(&total, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) P.state->n_tokens = total;
+}
+
+// For a tie: every pair's count and first position (tile * kTile + place), in dump_counts / dump_first by symbol numbers.
+__global__ void __launch_bounds__(kTileThreads) tile_dump_kernel(const TileParams P, uint32_t buffer) {
+    CHKRP_DYN_SMEM(smem);
+    TileCountSmem* const cs = reinterpret_cast<TileCountSmem*>(smem);
+    const uint32_t t = blockIdx.x, tid = threadIdx.x, side = P.state->side, n_symbols = P.state->n_symbols;
+    uint32_t* const counts = cs->pairs;
+    uint32_t* const first = cs->pairs + side * side;
+    tile_load_numbers(P, cs);
+    for (uint32_t i = tid; i < side * side; i += kTileThreads) {
+        counts[i] = 0;
+        first[i] = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    const TileEnds* const e = buffer ? P.ends[1] : P.ends[0];
+    const uint32_t len = e[t].len;
+    const uint16_t* const in = (buffer ? P.tokens[1] : P.tokens[0]) + (size_t)t * kTile;
+    for (uint32_t i = tid; i < len; i += kTileThreads) {
+        uint32_t r = 0;
+        if (i + 1 < len)
+            r = in[i + 1];
+        else if (!tile_next_first(e, P.n_tiles, t, &r))
+            continue;
+        const uint32_t at = symbol_of_token(cs, n_symbols, in[i]) * side + symbol_of_token(cs, n_symbols, r);
+        atomicAdd(&counts[at], 1u);
+        atomicMin(&first[at], t * kTile + i);
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < side * side; i += kTileThreads)
+        if (counts[i]) {
+            atomicAdd(&P.dump_counts[i], counts[i]);
+            atomicMin(&P.dump_first[i], first[i]);
+        }
 }
 
 }  // namespace chkrp

@@ -139,3 +139,64 @@ int emu_clusters(size_t n, const char* const* names, const float* fps, int32_t* 
 }
 
 }  // extern "C"
+
+// ---------------------------------------------------------------- Re-Pair on tiles
+#include "repair_kernels.cuh"
+
+extern "C" {
+
+// n words (nothing masked) through the tile kernels.  count: words, pairs, then rules 0 .. n_rules - 1 are chosen and
+// applied as far as they go (the last one without counting); else the rules given are applied.  out: the final tokens;
+// state_out: RoundState; on a tie dump_* (side * side) and word_of.  Returns the number of tokens in `out`.
+uint32_t emu_tile_rounds(const uint32_t* words, uint32_t n, uint32_t n_rules, uint32_t count, uint32_t* rules, uint16_t* out,
+                         uint32_t* state_out, uint32_t* dump_counts, uint32_t* dump_first, uint16_t* word_of) {
+    using namespace chkrp;
+    TileParams P{};
+    P.n_tiles = (n + kTile - 1) / kTile;
+    P.max_rules = n_rules;
+    std::vector<uint16_t> a(P.n_tiles * kTile, 0xDEAD), b(P.n_tiles * kTile, 0xDEAD);
+    std::vector<uint8_t> present(1u << kTileBits, 0), number(1u << kTileBits, 0xCD);
+    std::vector<uint32_t> freq(n_rules + 1), pairs(kDense * kDense, 0);
+    std::vector<TileEnds> e0(P.n_tiles), e1(P.n_tiles);
+    std::vector<uint2> r(n_rules + 1);
+    for (uint32_t i = 0; i < n_rules; ++i) r[i] = make_uint2(rules[2 * i], rules[2 * i + 1]);
+    RoundState st{};
+    P.tokens[0] = a.data(); P.tokens[1] = b.data();
+    P.ends[0] = e0.data(); P.ends[1] = e1.data();
+    P.rules = r.data(); P.rule_freq = freq.data(); P.state = &st;
+    P.present = present.data(); P.number = number.data(); P.word_of = word_of; P.pairs = pairs.data();
+    P.dump_counts = dump_counts; P.dump_first = dump_first;
+    uint32_t current = 0;
+    const auto raw = (const uint8_t*)words;
+    if (count) {
+        emu::launch(P.n_tiles, kTileThreads, sizeof(TileCountSmem), [&] { tile_words_kernel<true>(raw, n, 4, 0, P); });
+        emu::launch(P.n_tiles, kTileThreads, tile_count_smem(kDense), [&] { tile_pairs_kernel(P); });
+    } else {
+        emu::launch(P.n_tiles, kTileThreads, sizeof(TileCountSmem), [&] { tile_words_kernel<false>(raw, n, 4, 0, P); });
+    }
+    for (uint32_t k = 0; k < n_rules; ++k) {
+        if (st.stop != kGoOn) break;
+        if (count && k + 1 < n_rules)
+            emu::launch(P.n_tiles, kTileThreads, tile_count_smem(st.side), [&] { tile_rule_kernel<true>(P, k); });
+        else
+            emu::launch(P.n_tiles, kTileThreads, sizeof(TileCountSmem), [&] { tile_rule_kernel<false>(P, k); });
+        current = 1 - current;
+    }
+    emu::launch(1, kTileThreads, 0, [&] { tile_total_kernel(P, current); });
+    if (st.stop == kTie) {
+        std::fill(dump_counts, dump_counts + st.side * st.side, 0u);
+        std::fill(dump_first, dump_first + st.side * st.side, 0xFFFFFFFFu);
+        emu::launch(P.n_tiles, kTileThreads, tile_count_smem(st.side) + st.side * st.side * 4, [&] { tile_dump_kernel(P, current); });
+    }
+    uint32_t at = 0;
+    for (uint32_t t = 0; t < P.n_tiles; ++t)
+        for (uint32_t i = 0; i < P.ends[current][t].len; ++i) out[at++] = P.tokens[current][t * kTile + i];
+    for (uint32_t i = 0; i < n_rules; ++i) {
+        rules[2 * i] = r[i].x;
+        rules[2 * i + 1] = r[i].y;
+    }
+    std::memcpy(state_out, &st, sizeof(st));
+    return at;
+}
+
+}  // extern "C"

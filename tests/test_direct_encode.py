@@ -257,6 +257,83 @@ def test_clusters_as_the_oracle_forms_them(direct_lib, oracle, n, kind):
         assert k == len(anchors) and np.array_equal(ids, want)
 
 
+def _tile_rounds(lib, words, rules, n_rules, count):
+    n, dense = words.size, 144
+    r = np.zeros((max(n_rules, 1), 2), np.uint32)
+    r[:len(rules)] = np.reshape(rules, (-1, 2))
+    out, state = np.zeros(n, np.uint16), np.zeros(9, np.uint32)
+    dc, df, wo = np.zeros(dense * dense, np.uint32), np.zeros(dense * dense, np.uint32), np.zeros(dense, np.uint16)
+    lib.emu_tile_rounds.restype = C.c_uint32
+    u16p = C.POINTER(C.c_uint16)
+    m = lib.emu_tile_rounds(words.ctypes.data_as(u32p), n, n_rules, int(count), r.ctypes.data_as(u32p), out.ctypes.data_as(u16p),
+                            state.ctypes.data_as(u32p), dc.ctypes.data_as(u32p), df.ctypes.data_as(u32p), wo.ctypes.data_as(u16p))
+    return [int(x) for x in out[:m]], state, r, dc, df, wo
+
+
+TILE = 4096
+
+
+def _tile_sequences():
+    rng = np.random.default_rng(8)
+    yield rng.integers(0, 3, 3 * TILE + 5)                             # runs and pairs across tile borders
+    yield np.zeros(2 * TILE + 1, np.int64)                             # one run through three tiles; the last can vanish
+    yield np.repeat(rng.integers(0, 2, 40), rng.integers(1, 700, 40))  # long runs, odd and even, over borders
+    yield rng.integers(0, 90, TILE + 1)                                # a last tile of one token
+    yield (np.abs(rng.normal(0, 3, 2 * TILE + 77)).astype(np.int64) + 4000)  # a few frequent words, wide ones
+    yield np.array([5])
+
+
+def test_repair_rules_on_tiles(direct_lib):
+    """Every rule over a few symbols, then rules over rule symbols, against the left-to-right rewrite."""
+    from test_repair import py_apply
+    for s in _tile_sequences():
+        t = np.ascontiguousarray(s, np.uint32)
+        vals = sorted(set(int(x) for x in t))[:3]
+        chains = [[(a, b)] for a in vals for b in vals] + [[(vals[0], vals[0]), (0x8000, 0x8000), (vals[-1], 0x8000), (0x8001, vals[0])]]
+        for rules in chains:
+            want = [int(x) for x in t]
+            for k, (a, b) in enumerate(rules):
+                want = py_apply(want, a, b, 0x8000 + k)
+            got, state, *_ = _tile_rounds(direct_lib, t, rules, len(rules), False)
+            assert got == want and state[2] == len(want), rules
+
+
+def test_repair_counts_on_tiles(direct_lib):
+    """The rule picked by each round, its count, and what is handed to the host when pairs tie."""
+    from test_repair import py_apply
+    for s in _tile_sequences():
+        t = np.ascontiguousarray(s, np.uint32)
+        n_rules = 12
+        got, state, rules, dc, df, wo = _tile_rounds(direct_lib, t, [], n_rules, True)
+        seq, k = [int(x) for x in t], 0
+        while True:
+            pairs = {}
+            for i in range(len(seq) - 1):
+                pairs.setdefault((seq[i], seq[i + 1]), []).append(i)
+            best = max((len(v) for v in pairs.values()), default=0)
+            top = [p for p, v in pairs.items() if len(v) == best]
+            if best < 2:
+                assert state[0] == 1
+                break
+            if len(top) > 1:
+                assert state[0] == 2
+                side, ns = int(state[7]), int(state[6])
+                token = lambda q: int(wo[q]) if q < ns else 0x8000 + q - ns  # noqa: E731
+                used = np.flatnonzero(dc[:side * side])
+                order = used[np.argsort(df[used])]
+                assert [(token(q // side), token(q % side)) for q in order] == list(pairs)
+                assert [int(x) for x in dc[order]] == [len(v) for v in pairs.values()]
+                break
+            assert tuple(int(x) for x in rules[k]) == top[0], (k, best)
+            k += 1
+            seq = py_apply(seq, *top[0], 0x8000 + k - 1)
+            if k == n_rules:
+                break
+        assert got == seq and state[2] == len(seq)
+    too_many = np.ascontiguousarray(np.random.default_rng(1).integers(0, 400, 9000), np.uint32)
+    assert _tile_rounds(direct_lib, too_many, [], 12, True)[1][0] == 3
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("workspace", [0, 1 << 20])
 def test_files_on_the_device(oracle, tmp_path, workspace):
