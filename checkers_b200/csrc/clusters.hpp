@@ -9,16 +9,16 @@
 // handed out in category-name order, then by union-find root.
 #pragma once
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <map>
 #include <numeric>
 #include <string>
-#include <thread>
 #include <unordered_map>
 #include <vector>
+
+#include "host_parallel.hpp"
 
 namespace chk {
 
@@ -33,25 +33,6 @@ inline const char* category_of_name(const std::string& name) {
     if (name.rfind("optimizer.exp_avg::", 0) == 0) return "exp_avg";
     if (name.rfind("master_weights::", 0) == 0) return "master_weights";
     return "model_state";
-}
-
-// f(0 .. n-1), on a few threads when the work is worth their start (tens of microseconds each).
-template <typename F>
-inline void cluster_parallel(size_t n, size_t work, F&& f) {
-    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t threads = std::min(std::min<size_t>(n, hw), std::min<size_t>(8, work / 50000 + 1));
-    if (threads <= 1) {
-        for (size_t i = 0; i < n; ++i) f(i);
-        return;
-    }
-    std::atomic<size_t> next{0};
-    auto run = [&] {
-        for (size_t i; (i = next.fetch_add(1)) < n;) f(i);
-    };
-    std::vector<std::thread> pool;
-    for (size_t k = 1; k < threads; ++k) pool.emplace_back(run);
-    run();
-    for (auto& t : pool) t.join();
 }
 
 // The element that sorting v (none negative) would leave at position `at`.  Doubles that are not negative order like
@@ -137,7 +118,7 @@ inline ClusterMap build_clusters(const std::vector<std::string>& names, const st
         cats.push_back(std::move(c));
     }
 
-    cluster_parallel(blocks.size(), pairs, [&](size_t i) {
+    host_parallel(blocks.size(), pairs, [&](size_t i) {
         const RowBlock& r = blocks[i];
         Category& c = cats[r.cat];
         const double* const p[5] = {c.at[0].data(), c.at[1].data(), c.at[2].data(), c.at[3].data(), c.at[4].data()};
@@ -157,7 +138,7 @@ inline ClusterMap build_clusters(const std::vector<std::string>& names, const st
     // so the quartile is the root of the quartile of the squares, and a distance lies below it exactly when its square
     // lies below the smallest number whose root is the threshold.  Once everything is in one set, no pair changes
     // anything any more.
-    cluster_parallel(cats.size(), pairs, [&](size_t i) {
+    host_parallel(cats.size(), pairs, [&](size_t i) {
         Category& c = cats[i];
         DisjointSet ds(c.m);
         if (!c.squared.empty()) {

@@ -1,0 +1,77 @@
+// host_parallel.hpp -- loops of the host code spread over a few threads, and an index of names.
+#pragma once
+#include <algorithm>
+#include <atomic>
+#include <cstddef>
+#include <cstdint>
+#include <functional>
+#include <string_view>
+#include <system_error>
+#include <thread>
+#include <vector>
+
+namespace chk {
+
+// f(0 .. n-1), on a few threads when the work (in nanoseconds, roughly) is worth their start (tens of microseconds each).
+template <typename F>
+inline void host_parallel(size_t n, size_t work, F&& f) {
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t threads = std::min(std::min<size_t>(n, hw), std::min<size_t>(8, work / 50000 + 1));
+    if (threads <= 1) {
+        for (size_t i = 0; i < n; ++i) f(i);
+        return;
+    }
+    std::atomic<size_t> next{0};
+    auto run = [&] {
+        for (size_t i; (i = next.fetch_add(1)) < n;) f(i);
+    };
+    std::vector<std::thread> pool;
+    try {
+        for (size_t k = 1; k < threads; ++k) pool.emplace_back(run);
+    } catch (const std::system_error&) {
+        // no more threads to be had: those there are do it all
+    }
+    run();
+    for (auto& t : pool) t.join();
+}
+
+// Name -> position, the first one where a name occurs twice.  The names stay where they are (key(i) says where): one
+// flat array of hash tags and positions, so neither building it nor asking it allocates per name, and a name's own
+// memory is touched only when its tag matches.
+class NameIndex {
+   public:
+    static constexpr size_t kNone = ~(size_t)0;
+    template <typename Key>
+    void build(size_t n, const Key& key) {
+        size_t cap = 16;
+        while (cap < 2 * n) cap *= 2;
+        mask_ = cap - 1;
+        slots_.assign(cap, Slot{0, kEmpty});
+        for (size_t i = 0; i < n; ++i) {
+            const std::string_view name = key(i);
+            const size_t h = std::hash<std::string_view>{}(name);
+            size_t p = h & mask_;
+            for (; slots_[p].at != kEmpty; p = (p + 1) & mask_)
+                if (slots_[p].tag == tag(h) && key(slots_[p].at) == name) break;
+            if (slots_[p].at == kEmpty) slots_[p] = Slot{tag(h), (uint32_t)i};
+        }
+    }
+    template <typename Key>
+    size_t find(std::string_view name, const Key& key) const {
+        const size_t h = std::hash<std::string_view>{}(name);
+        for (size_t p = h & mask_; slots_[p].at != kEmpty; p = (p + 1) & mask_)
+            if (slots_[p].tag == tag(h) && key(slots_[p].at) == name) return slots_[p].at;
+        return kNone;
+    }
+
+   private:
+    static constexpr uint32_t kEmpty = ~0u;
+    struct Slot {
+        uint32_t tag, at;
+    };
+    static uint32_t tag(size_t h) { return (uint32_t)(h >> 32); }
+    std::vector<Slot> slots_;
+    size_t mask_ = 0;
+};
+
+}  // namespace chk

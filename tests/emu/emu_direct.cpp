@@ -138,6 +138,14 @@ int emu_clusters(size_t n, const char* const* names, const float* fps, int32_t* 
     return m.n_clusters;
 }
 
+// NameIndex over `names`, asked for every one of `asked` (~0: not there), by several threads.
+void emu_name_index(size_t n, const char* const* names, size_t n_asked, const char* const* asked, uint64_t* at) {
+    auto key = [&](size_t i) { return std::string_view(names[i]); };
+    NameIndex index;
+    index.build(n, key);
+    host_parallel(n_asked, 1u << 20, [&](size_t i) { at[i] = index.find(asked[i], key); });
+}
+
 }  // extern "C"
 
 // ---------------------------------------------------------------- Re-Pair on tiles

@@ -334,6 +334,54 @@ def test_repair_counts_on_tiles(direct_lib):
     assert _tile_rounds(direct_lib, too_many, [], 12, True)[1][0] == 3
 
 
+@pytest.mark.parametrize("n", [0, 1, 8, 9, 1000])
+def test_name_index_finds_the_first_of_equal_names(direct_lib, n):
+    names = [f"layer.{i % max(1, n - n // 4)}" for i in range(n)]
+    asked = names + ["", "layer.", "layer.1000"]
+    first = {}
+    for i, nm in enumerate(names):
+        first.setdefault(nm, i)
+    arr = lambda v: (C.c_char_p * max(1, len(v)))(*[x.encode() for x in v])
+    at = (C.c_uint64 * len(asked))()
+    direct_lib.emu_name_index(C.c_size_t(n), arr(names), C.c_size_t(len(asked)), arr(asked), at)
+    assert list(at) == [first.get(nm, 2**64 - 1) for nm in asked]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [63, 64, 65, 700])
+def test_index_of_many_entries_on_the_device(oracle, tmp_path, n):
+    """Entries are written and read in pieces of 64: the oracle's files, a restore that has it all, and of two damaged
+    entries in two pieces the first one is named."""
+    torch = pytest.importorskip("torch")
+    import checkers_b200 as chk
+    host = [synth("i8" if i % 5 == 4 else "f32_master", 300 + i, i) for i in range(n)]
+    names = [f"t{i}" for i in range(n)]
+    dev = [torch.from_numpy(raw.copy()).cuda() for raw, _ in host]
+    torch.cuda.synchronize()
+    ctx = chk.Context(device=0)
+    for nm, d, (raw, dt) in zip(names, dev, host):
+        ctx.register_pointer(nm, d.data_ptr(), raw.size // ELEM_SIZE[dt], dt)
+    ctx.compress_and_save(str(tmp_path / "gpu"))
+    oracle.compress_and_save(names, [r for r, _ in host], [d for _, d in host], str(tmp_path / "cpu"))
+    images = []
+    for rel in ("rank_0_states.ansc", "mantissa/rank_0_mantissa.mant", "tables/rank_0_tables.dict"):
+        images.append(np.fromfile(tmp_path / "gpu" / rel, np.uint8))
+        assert np.array_equal(images[-1], np.fromfile(tmp_path / "cpu" / rel, np.uint8)), rel
+    for d in dev:
+        d.zero_()
+    torch.cuda.synchronize()
+    assert ctx.decompress_images(*images) == n
+    for d, (raw, _) in zip(dev, host):
+        assert np.array_equal(d.cpu().numpy(), raw)
+    bad = images[0].copy()
+    for i, lane in ((n - 1, 3), (n // 2, 200)):  # an entry takes 4648 bytes; lane header: state, byte count, offset, padding
+        bad[16 + i * 4648 + 257] = 0  # coded, whatever it was
+        bad[16 + i * 4648 + 552 + 16 * lane + 4:][:4] = 255
+    with pytest.raises(chk.CheckersError, match=f"entry 't{n // 2}': lane 200 out of range"):
+        ctx.decompress_images(bad, *images[1:])
+    ctx.close()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("workspace", [0, 1 << 20])
 def test_files_on_the_device(oracle, tmp_path, workspace):
