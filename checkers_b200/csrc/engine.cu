@@ -427,7 +427,7 @@ static void compress(Context* c, bool host_images) {
     pin_ensure(c->h_tiles, (W + 1) * 4);
     uint32_t* tile_start = static_cast<uint32_t*>(c->h_tiles.p);
     tile_start[0] = 0;
-    unsigned long long sidecar_total = 0, bytes_total = 0, slot_bytes = 0, regions_total = 0;
+    unsigned long long sidecar_total = 0, bytes_total = 0, ragged_bytes = 0, slot_bytes = 0, regions_total = 0;
     uint32_t max_stride = 0;
     size_t n_sidecars = 0;
     bool any_member = false, any_int = false;
@@ -445,7 +445,10 @@ static void compress(Context* c, bool host_images) {
         d.chunk_stride = (uint32_t)((2 * c_max + 31) & ~31ull);
         d.flags = w.owns ? kFlagNeedHist : 0u;
         if (c->tensors[w.idx].hot) d.flags |= kFlagHotBins;
-        if ((reinterpret_cast<uintptr_t>(d.src) & 15) == 0 && (sidecar_total & 15) == 0) d.flags |= kFlagAligned;
+        if ((reinterpret_cast<uintptr_t>(d.src) & 15) == 0 && (sidecar_total & 15) == 0)
+            d.flags |= kFlagAligned;
+        else
+            ragged_bytes += w.bytes;
         sidecar_total += (unsigned long long)c->tensors[w.idx].n_elem * w.spe;
         // value-lane regions, plus one shared region for the lanes that only see zeroed bytes
         const unsigned long long need = (w.spe * 2 == w.es ? 129ull : 256ull) * d.chunk_stride;
@@ -602,10 +605,10 @@ static void compress(Context* c, bool host_images) {
         const uint32_t tiles = tile_start[b] - tile_start[a];
         const uint32_t grid1 = tiles < sms * 8u ? tiles : sms * 8u;
         if (!c->precounted) {
-            split_hist_kernel<<<grid1, 256, 0, s>>>(static_cast<const TensorDesc*>(c->d_descs.p) + a,
-                                                    static_cast<const uint32_t*>(c->d_tiles.p) + a, (uint32_t)n, tile_start[a],
-                                                    tiles, static_cast<uint8_t*>(c->d_sidecar.p),
-                                                    static_cast<uint32_t*>(c->d_hist.p) + a * 256);
+            const auto split = ragged_split_pays(ragged_bytes, bytes_total) ? split_ragged_kernel : split_hist_kernel;
+            split<<<grid1, 256, 0, s>>>(static_cast<const TensorDesc*>(c->d_descs.p) + a,
+                                        static_cast<const uint32_t*>(c->d_tiles.p) + a, (uint32_t)n, tile_start[a], tiles,
+                                        static_cast<uint8_t*>(c->d_sidecar.p), static_cast<uint32_t*>(c->d_hist.p) + a * 256);
             CHK_CUDA(cudaGetLastError());
             c->launches++;
         }

@@ -138,6 +138,24 @@ int emu_clusters(size_t n, const char* const* names, const float* fps, int32_t* 
     return m.n_clusters;
 }
 
+// split_ragged_kernel over n tensors; sidecar (null: count only) takes the low bytes from side_off[i] on.
+void emu_split_ragged(size_t n, const uint8_t* const* srcs, const uint64_t* n_bytes, const uint32_t* es, const uint32_t* spe,
+                      const uint64_t* side_off, uint8_t* sidecar, uint32_t* hist, uint32_t grid) {
+    std::vector<TensorDesc> descs(n);
+    std::vector<uint32_t> tiles(n + 1, 0);
+    for (size_t i = 0; i < n; ++i) {
+        std::memset(&descs[i], 0, sizeof(TensorDesc));
+        descs[i].src = srcs[i];
+        descs[i].n_bytes = n_bytes[i];
+        descs[i].es = es[i];
+        descs[i].spe = spe[i];
+        descs[i].sidecar_off = side_off[i];
+        descs[i].flags = kFlagNeedHist;
+        tiles[i + 1] = tiles[i] + (uint32_t)((n_bytes[i] + kSplitTileBytes - 1) / kSplitTileBytes);
+    }
+    emu::launch(grid, 256, 0, [&] { split_ragged_kernel(descs.data(), tiles.data(), (uint32_t)n, 0u, tiles[n], sidecar, hist); });
+}
+
 // NameIndex over `names`, asked for every one of `asked` (~0: not there), by several threads.
 void emu_name_index(size_t n, const char* const* names, size_t n_asked, const char* const* asked, uint64_t* at) {
     auto key = [&](size_t i) { return std::string_view(names[i]); };

@@ -334,6 +334,41 @@ def test_repair_counts_on_tiles(direct_lib):
     assert _tile_rounds(direct_lib, too_many, [], 12, True)[1][0] == 3
 
 
+@pytest.mark.parametrize("es,spe", [(4, 2), (2, 1), (4, 0), (1, 0)])
+@pytest.mark.parametrize("at", range(0, 16, 3))
+def test_split_of_tensors_at_any_address(direct_lib, es, spe, at):
+    """Sources and low bytes at every alignment: the low bytes in place, nothing beside them, all other bytes counted."""
+    rng = np.random.default_rng(es * 16 + at)
+    sizes = [es * k for k in (1, 3, 7, 16, 17, 40)] + [4096 - es, 4096 + 5 * es, 32768, 32768 + es, 70000]
+    tensors = [rng.integers(0, 256, n, np.uint8) for n in sizes]
+    space = [aligned(n + 64) for n in sizes]
+    srcs = []
+    for i, (t, b) in enumerate(zip(tensors, space)):
+        o = (at + es * i) % 16
+        b[o:o + t.size] = t
+        srcs.append(b.ctypes.data + o)
+    gap, off = 5, []
+    total = 32 + at
+    for n in sizes:
+        off.append(total)
+        total += n // es * spe + gap
+    low = aligned(total + 64)
+    low[:] = 0xA5
+    want = low.copy()
+    hist = np.zeros((len(sizes), 256), np.uint32)
+    ref = np.zeros_like(hist)
+    for i, t in enumerate(tensors):
+        e = t.reshape(-1, es)
+        want[off[i]:off[i] + e.shape[0] * spe] = e[:, :spe].reshape(-1)
+        ref[i] = np.bincount(e[:, spe:].reshape(-1), minlength=256)
+    n = len(sizes)
+    direct_lib.emu_split_ragged(C.c_size_t(n), (C.c_void_p * n)(*srcs), (C.c_uint64 * n)(*sizes), (C.c_uint32 * n)(*[es] * n),
+                                (C.c_uint32 * n)(*[spe] * n), (C.c_uint64 * n)(*off), C.c_void_p(low.ctypes.data),
+                                hist.ctypes.data_as(C.c_void_p), C.c_uint32(3))
+    assert np.array_equal(low, want)
+    assert np.array_equal(hist, ref)
+
+
 @pytest.mark.parametrize("n", [0, 1, 8, 9, 1000])
 def test_name_index_finds_the_first_of_equal_names(direct_lib, n):
     names = [f"layer.{i % max(1, n - n // 4)}" for i in range(n)]
