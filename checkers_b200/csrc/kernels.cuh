@@ -130,11 +130,56 @@ __device__ __forceinline__ void split_one_byte(const TensorDesc& d, unsigned lon
     }
 }
 
+// Consecutive pieces of a byte stream, one per lane (4 or 8 bytes each), that land `shift` bytes past a word boundary: each
+// lane stores the whole word its piece starts in, with the end of the neighbouring lane's piece.  Only the two ends of the
+// stretch that a warp stores go byte by byte: the first piece (`first`), and the end of the last one (finish).
+__device__ __forceinline__ uint8_t piece_byte(uint32_t w, uint32_t j) { return (uint8_t)(w >> (8 * j)); }
+__device__ __forceinline__ uint8_t piece_byte(uint2 w, uint32_t j) { return piece_byte(j < 4 ? w.x : w.y, j & 3); }
+__device__ __forceinline__ uint32_t piece_neighbour(uint32_t own, uint32_t& before, uint32_t lane) {
+    const uint32_t p = __shfl_up_sync(0xFFFFFFFFu, own, 1), b = before;
+    before = __shfl_sync(0xFFFFFFFFu, own, 31);
+    return lane ? p : b;
+}
+__device__ __forceinline__ uint2 piece_neighbour(uint2 own, uint2& before, uint32_t lane) {
+    return make_uint2(piece_neighbour(own.x, before.x, lane), piece_neighbour(own.y, before.y, lane));
+}
+__device__ __forceinline__ uint32_t piece_word(uint32_t p, uint32_t own, uint32_t shift) {
+    return __funnelshift_l(p, own, shift * 8);
+}
+__device__ __forceinline__ uint2 piece_word(uint2 p, uint2 own, uint32_t shift) {
+    const uint32_t a0 = shift & 4 ? p.x : p.y, a1 = shift & 4 ? p.y : own.x, a2 = shift & 4 ? own.x : own.y;
+    return make_uint2(__funnelshift_l(a0, a1, (shift & 3) * 8), __funnelshift_l(a1, a2, (shift & 3) * 8));
+}
+template <typename Piece>
+struct ShiftedStore {
+    Piece before, last;
+    uint32_t shift;
+    __device__ __forceinline__ explicit ShiftedStore(const uint8_t* at)
+        : before(), last(), shift((uint32_t)(uintptr_t)at & (uint32_t)(sizeof(Piece) - 1)) {}
+    // every lane of the warp comes here; `at`: where the piece starts, if `valid`
+    __device__ __forceinline__ void put(uint8_t* at, Piece own, bool valid, bool first, uint32_t lane) {
+        if (!shift) {
+            if (valid) *reinterpret_cast<Piece*>(at) = own;
+            return;
+        }
+        const Piece p = piece_neighbour(own, before, lane);
+        if (!valid) return;
+        last = own;
+        if (first)
+            for (uint32_t j = 0; j < sizeof(Piece) - shift; ++j) at[j] = piece_byte(own, j);
+        else
+            *reinterpret_cast<Piece*>(at - shift) = piece_word(p, own, shift);
+    }
+    // by the lane whose put was the stretch's last valid one
+    __device__ __forceinline__ void finish(uint8_t* at) const {
+        for (uint32_t j = (uint32_t)sizeof(Piece) - shift; j < sizeof(Piece); ++j) at[j] = piece_byte(last, j);
+    }
+};
+
 // A tile (its first nb bytes at tensor offset `base`) of a tensor whose bytes or low bytes need not start on a 16-byte
 // boundary, as the slices of a flat buffer at odd element counts do.  The source is read in 16-byte vectors from its
-// first 16-byte boundary on; the bytes before it and after the last whole vector go one by one.  Low bytes that start
-// inside an 8-byte word are shifted to the word's boundary with the end of the neighbouring lane's: each warp takes a
-// stretch of consecutive vectors, so only the ends of the stretch are written byte by byte.
+// first 16-byte boundary on; the bytes before it and after the last whole vector go one by one.  Each warp takes a
+// stretch of consecutive vectors, for the sake of low bytes that start inside an 8-byte word (ShiftedStore).
 __device__ __forceinline__ void split_ragged_tile(const TensorDesc& d, unsigned long long base, uint32_t nb,
                                                   uint8_t* __restrict__ sidecar, uint32_t* mine, uint32_t* mine_hot) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -175,8 +220,7 @@ __device__ __forceinline__ void split_ragged_tile(const TensorDesc& d, unsigned 
         if (v0 + u * 32 < nvec) q[u] = ld_global_v4(src + head + (size_t)(v0 + u * 32) * 16);
     }
     uint8_t* const side = sidecar ? sidecar + d.sidecar_off + ((base + head) >> 1) : nullptr;
-    const uint32_t shift = (uint32_t)(uintptr_t)side & 7u;  // the same for every vector
-    uint2 before = make_uint2(0, 0), last = before;         // lane 0: the low bytes of the vector before its own
+    ShiftedStore<uint2> out(side);
 #pragma unroll
     for (int u = 0; u < kSplitLoads; ++u) {
         const uint32_t v = v0 + u * 32;
@@ -190,28 +234,8 @@ __device__ __forceinline__ void split_ragged_tile(const TensorDesc& d, unsigned 
             own.x = __byte_perm(w[0], w[1], 0x6420);
             own.y = __byte_perm(w[2], w[3], 0x6420);
         }
-        uint8_t* const at = side + (size_t)v * 8;
-        if (shift) {
-            // what goes to the 8-byte word in which these low bytes start: the end of the vector before, then these
-            uint2 p;
-            p.x = __shfl_up_sync(0xFFFFFFFFu, own.x, 1);
-            p.y = __shfl_up_sync(0xFFFFFFFFu, own.y, 1);
-            if (lane == 0) p = before;
-            before.x = __shfl_sync(0xFFFFFFFFu, own.x, 31);
-            before.y = __shfl_sync(0xFFFFFFFFu, own.y, 31);
-            if (v >= nvec) continue;
-            last = own;
-            const uint32_t bits = (shift & 3) * 8;
-            const uint32_t a0 = shift & 4 ? p.x : p.y, a1 = shift & 4 ? p.y : own.x, a2 = shift & 4 ? own.x : own.y;
-            if (u == 0 && lane == 0)
-                for (uint32_t j = 0; j < 8 - shift; ++j) at[j] = (uint8_t)((j < 4 ? own.x : own.y) >> (8 * (j & 3)));
-            else
-                *reinterpret_cast<uint2*>(at - shift) = make_uint2(__funnelshift_l(a0, a1, bits), __funnelshift_l(a1, a2, bits));
-        } else {
-            if (v >= nvec) continue;
-            if (side) *reinterpret_cast<uint2*>(at) = own;
-        }
-        if (!count) continue;
+        if (side) out.put(side + (size_t)v * 8, own, v < nvec, u == 0 && lane == 0, lane);
+        if (!count || v >= nvec) continue;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (d.es == 4)
@@ -221,10 +245,7 @@ __device__ __forceinline__ void split_ragged_tile(const TensorDesc& d, unsigned 
             bin_add_hot(mine_hot, w[k] >> 24);
         }
     }
-    // the end of the warp's last vector starts a word that no vector of this warp completes
-    if (shift && end > first && ((end - 1 - first) & 31) == lane)
-        for (uint32_t j = 8 - shift; j < 8; ++j)
-            side[(size_t)(end - 1) * 8 + j] = (uint8_t)((j < 4 ? last.x : last.y) >> (8 * (j & 3)));
+    if (side && end > first && ((end - 1 - first) & 31) == lane) out.finish(side + (size_t)(end - 1) * 8);
 }
 
 // Fused row-1 + row-2 pass over all tensors of a batch: writes each tensor's

@@ -156,6 +156,26 @@ void emu_split_ragged(size_t n, const uint8_t* const* srcs, const uint64_t* n_by
     emu::launch(grid, 256, 0, [&] { split_ragged_kernel(descs.data(), tiles.data(), (uint32_t)n, 0u, tiles[n], sidecar, hist); });
 }
 
+// plane_split_ragged_kernel (hist: the counting one, 256 counters per plane) over n tensors
+void emu_planes_ragged(size_t n, uint8_t* const* srcs, const uint64_t* n_bytes, const uint32_t* es, const uint32_t* spe,
+                       const uint64_t* low_off, const uint64_t* plane_off, const uint64_t* stride, uint8_t* low, uint8_t* planes,
+                       uint32_t* hist, uint32_t grid) {
+    std::vector<PlaneDesc> d(n);
+    std::vector<uint32_t> tiles(n + 1, 0);
+    uint32_t row = 0;
+    for (size_t i = 0; i < n; ++i) {
+        d[i] = PlaneDesc{srcs[i], n_bytes[i] / es[i], low_off[i], plane_off[i], stride[i], es[i], spe[i], 0u, row};
+        row += es[i] - spe[i];
+        tiles[i + 1] = tiles[i] + (uint32_t)((n_bytes[i] + kPlaneTileBytes - 1) / kPlaneTileBytes);
+    }
+    emu::launch(grid, 256, hist ? kPlaneCountSmem + 128 : 0, [&] {
+        if (hist)
+            plane_split_count_ragged_kernel(d.data(), tiles.data(), (uint32_t)n, tiles[n], low, planes, hist);
+        else
+            plane_split_ragged_kernel(d.data(), tiles.data(), (uint32_t)n, tiles[n], low, planes);
+    });
+}
+
 // NameIndex over `names`, asked for every one of `asked` (~0: not there), by several threads.
 void emu_name_index(size_t n, const char* const* names, size_t n_asked, const char* const* asked, uint64_t* at) {
     auto key = [&](size_t i) { return std::string_view(names[i]); };

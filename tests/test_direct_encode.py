@@ -334,39 +334,65 @@ def test_repair_counts_on_tiles(direct_lib):
     assert _tile_rounds(direct_lib, too_many, [], 12, True)[1][0] == 3
 
 
-@pytest.mark.parametrize("es,spe", [(4, 2), (2, 1), (4, 0), (1, 0)])
-@pytest.mark.parametrize("at", range(0, 16, 3))
-def test_split_of_tensors_at_any_address(direct_lib, es, spe, at):
-    """Sources and low bytes at every alignment: the low bytes in place, nothing beside them, all other bytes counted."""
+def _at_any_address(es, spe, at):
+    """Tensors around the sizes of vectors, a warp's stretch and a tile, at every alignment; where their low bytes go."""
     rng = np.random.default_rng(es * 16 + at)
     sizes = [es * k for k in (1, 3, 7, 16, 17, 40)] + [4096 - es, 4096 + 5 * es, 32768, 32768 + es, 70000]
     tensors = [rng.integers(0, 256, n, np.uint8) for n in sizes]
-    space = [aligned(n + 64) for n in sizes]
-    srcs = []
-    for i, (t, b) in enumerate(zip(tensors, space)):
+    space, srcs, off, total = [], [], [], 32 + at
+    for i, t in enumerate(tensors):
+        space.append(aligned(t.size + 64))
         o = (at + es * i) % 16
-        b[o:o + t.size] = t
-        srcs.append(b.ctypes.data + o)
-    gap, off = 5, []
-    total = 32 + at
-    for n in sizes:
+        space[-1][o:o + t.size] = t
+        srcs.append(space[-1].ctypes.data + o)
         off.append(total)
-        total += n // es * spe + gap
+        total += t.size // es * spe + 5
     low = aligned(total + 64)
     low[:] = 0xA5
     want = low.copy()
-    hist = np.zeros((len(sizes), 256), np.uint32)
-    ref = np.zeros_like(hist)
-    for i, t in enumerate(tensors):
-        e = t.reshape(-1, es)
-        want[off[i]:off[i] + e.shape[0] * spe] = e[:, :spe].reshape(-1)
-        ref[i] = np.bincount(e[:, spe:].reshape(-1), minlength=256)
+    for t, o in zip(tensors, off):
+        e = t.reshape(-1, es)[:, :spe]
+        want[o:o + e.size] = e.reshape(-1)
     n = len(sizes)
-    direct_lib.emu_split_ragged(C.c_size_t(n), (C.c_void_p * n)(*srcs), (C.c_uint64 * n)(*sizes), (C.c_uint32 * n)(*[es] * n),
-                                (C.c_uint32 * n)(*[spe] * n), (C.c_uint64 * n)(*off), C.c_void_p(low.ctypes.data),
-                                hist.ctypes.data_as(C.c_void_p), C.c_uint32(3))
+    args = [C.c_size_t(n), (C.c_void_p * n)(*srcs), (C.c_uint64 * n)(*sizes), (C.c_uint32 * n)(*[es] * n),
+            (C.c_uint32 * n)(*[spe] * n), (C.c_uint64 * n)(*off)]
+    return [t.reshape(-1, es) for t in tensors], space, args, low, want
+
+
+@pytest.mark.parametrize("es,spe", [(4, 2), (2, 1), (4, 0), (1, 0)])
+@pytest.mark.parametrize("at", range(0, 16, 3))
+def test_split_of_tensors_at_any_address(direct_lib, es, spe, at):
+    """The low bytes in place, nothing beside them, all other bytes counted."""
+    tensors, space, args, low, want = _at_any_address(es, spe, at)
+    hist = np.zeros((len(tensors), 256), np.uint32)
+    ref = np.stack([np.bincount(t[:, spe:].reshape(-1), minlength=256) for t in tensors])
+    direct_lib.emu_split_ragged(*args, C.c_void_p(low.ctypes.data), hist.ctypes.data_as(C.c_void_p), C.c_uint32(3))
     assert np.array_equal(low, want)
     assert np.array_equal(hist, ref)
+
+
+@pytest.mark.parametrize("es", [4, 2])
+@pytest.mark.parametrize("count", [True, False])
+@pytest.mark.parametrize("at", range(0, 16, 3))
+def test_planes_of_tensors_at_any_address(direct_lib, es, count, at):
+    tensors, space, args, low, want = _at_any_address(es, es // 2, at)
+    n, k = len(tensors), es - es // 2
+    stride = [-(-t.shape[0] // 32) * 32 for t in tensors]
+    plane_off = [int(x) for x in np.cumsum([0] + [k * s for s in stride])]
+    planes = aligned(plane_off[-1] + 64)
+    planes[:] = 0x5A
+    want_planes = planes.copy()
+    for t, s, o in zip(tensors, stride, plane_off):
+        for j in range(k):
+            want_planes[o + j * s:o + j * s + t.shape[0]] = t[:, es // 2 + j]
+    hist = np.zeros((n * k, 256), np.uint32)
+    ref = np.concatenate([[np.bincount(t[:, es // 2 + j], minlength=256) for j in range(k)] for t in tensors])
+    direct_lib.emu_planes_ragged(*args, (C.c_uint64 * n)(*plane_off[:-1]), (C.c_uint64 * n)(*stride),
+                                 C.c_void_p(low.ctypes.data), C.c_void_p(planes.ctypes.data),
+                                 hist.ctypes.data_as(C.c_void_p) if count else None, C.c_uint32(3))
+    assert np.array_equal(low, want)
+    assert np.array_equal(planes, want_planes)
+    assert not count or np.array_equal(hist, ref)
 
 
 @pytest.mark.parametrize("n", [0, 1, 8, 9, 1000])
