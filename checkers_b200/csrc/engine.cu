@@ -2076,21 +2076,29 @@ namespace chk {
 constexpr unsigned long long kStaticMaxTensorBytes = CHK_STATIC_MAX_TENSOR_BYTES;
 constexpr uint32_t kStaticChunkStride = (uint32_t)(2 * ((kStaticMaxTensorBytes + 255) / 256));  // bytes per lane
 
-struct StaticScratch {
+struct StaticHead {  // set by every call
     TensorDesc desc;
-    uint32_t order[4];
-    uint32_t ticket[4];
-    unsigned long long payload_size[2];
-    unsigned long long payload_off[2];
-    EncEntry enc[256];
+    unsigned long long payload_size;
+    uint32_t ticket, done;  // start at zero
+    uint32_t order[2];
+    uint32_t items[2];      // gather_lanes_kernel's pieces before and after the tensor
+    alignas(16) EncEntry enc[256];
+};
+struct StaticScratch {
+    StaticHead head;
     unsigned long long lane_src[256];
     uint32_t lane_off[256];
     alignas(256) uint8_t lanes[256ull * kStaticChunkStride + 256];  // lane regions are written 16 bytes at a time
 };
 constexpr size_t kStaticScratchBytes = sizeof(StaticScratch);
-static_assert(offsetof(StaticScratch, lanes) % 16 == 0 && offsetof(StaticScratch, lane_src) % 8 == 0 &&
-                  offsetof(StaticScratch, payload_size) % 8 == 0,
-              "static scratch members must keep their natural alignment");
+static_assert(offsetof(StaticScratch, lanes) % 16 == 0 && sizeof(StaticHead) % 16 == 0,
+              "static scratch members must keep their alignment");
+
+// The head travels as a kernel argument: no copy engine between the host and the first kernel, no staging buffer.
+__global__ void __launch_bounds__(256) static_head_kernel(const CHK_GRID_CONSTANT StaticHead head, StaticHead* __restrict__ dst) {
+    for (uint32_t i = threadIdx.x; i < sizeof(StaticHead) / 16; i += 256)
+        reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(&head)[i];
+}
 
 // In host code this name is only a handle for cudaGetSymbolAddress; the device
 // address it stands for is looked up once per device below.
@@ -2134,17 +2142,8 @@ extern "C" int chk_encode_tensor_static(const void* d_src, uint64_t num_elements
     StaticScratch* dev = reinterpret_cast<StaticScratch*>(base);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-    // host-side image of the small header part (desc .. enc); lives on this stack frame only
-    struct Head {
-        TensorDesc desc;
-        uint32_t order[4];
-        uint32_t ticket[4];
-        unsigned long long payload_size[2];
-        unsigned long long payload_off[2];
-        EncEntry enc[256];
-    } head;
-    static_assert(offsetof(StaticScratch, lane_src) == sizeof(Head), "header layout");
-    std::memset(&head, 0, sizeof(head));  // order[0] = 0, ticket = 0, sizes = 0
+    StaticHead head;
+    std::memset(&head, 0, sizeof(head));
     const unsigned long long c_max = (bytes + 255) / 256;
     head.desc.src = static_cast<const uint8_t*>(d_src);
     head.desc.n_bytes = bytes;
@@ -2153,6 +2152,7 @@ extern "C" int chk_encode_tensor_static(const void* d_src, uint64_t num_elements
     head.desc.table_idx = 0;
     head.desc.scratch_off = offsetof(StaticScratch, lanes);
     head.desc.chunk_stride = (uint32_t)((2 * c_max + 31) & ~31ull);
+    head.items[1] = kLanes * gather_pieces(bytes);
     CHK_REQUIRE(cum_freq[0] == 0, "cum_freq[0] must be 0");
     for (int i = 0; i < 256; ++i) {
         CHK_REQUIRE(norm_freq[i] <= kM, "norm_freq above 4096");
@@ -2166,31 +2166,43 @@ extern "C" int chk_encode_tensor_static(const void* d_src, uint64_t num_elements
     bool escape = false;
     for (int i = 0; i < 256 && !escape; ++i) escape = norm_freq[i] == 0;
 
-    // pageable source: the runtime stages it before returning, so the stack frame may go away
-    CHK_CUDA(cudaMemcpyAsync(base, &head, sizeof(head), cudaMemcpyHostToDevice, s));
+    // The direct path of compress() for a batch of one: the symbol-0 chain is a team beside the value lanes' (as a launch of
+    // its own before them it took a quarter of the call), and one copy brings the result back.  256 Ki bf16 elements take
+    // 174 us, with eight launches and copies in a row 244; 1 Mi fp32 elements 606 and 969; 1000 bf16 elements 54 and 83.
+    static_head_kernel<<<1, 256, 0, s>>>(head, &dev->head);
+    CHK_CUDA(cudaGetLastError());
     const bool ints = spe * 2 != es;
-    zero_lane_kernel<<<1, 32, 0, s>>>(&dev->desc, dev->enc, base, static_cast<LaneHeader*>(d_lane_headers), dev->lane_src,
-                                      1u);
+    LanesParams lp{};
+    lp.descs = &dev->head.desc;
+    lp.tables = dev->head.enc;
+    lp.scratch = base;
+    lp.hdrs = static_cast<LaneHeader*>(d_lane_headers);
+    lp.lane_src = dev->lane_src;
+    lp.order = dev->head.order;
+    lp.ticket = &dev->head.ticket;
+    lp.n_tensors = 1;
+    auto lanes = ints ? (escape ? rans_lanes_kernel<true, true> : rans_lanes_kernel<true, false>)
+                      : (escape ? rans_lanes_kernel<false, true> : rans_lanes_kernel<false, false>);
+    lanes<<<2, kTeam, ints ? sizeof(EncSmem<4>) : sizeof(EncSmem<2>), s>>>(lp);
     CHK_CUDA(cudaGetLastError());
-    auto kernel = ints ? (escape ? rans_encode_kernel<true, true> : rans_encode_kernel<true, false>)
-                       : (escape ? rans_encode_kernel<false, true> : rans_encode_kernel<false, false>);
-    kernel<<<1, kTeam, ints ? sizeof(EncSmem<4>) : sizeof(EncSmem<2>), s>>>(
-        &dev->desc, dev->enc, base, static_cast<LaneHeader*>(d_lane_headers), dev->lane_src, dev->order, dev->ticket, 1u);
+    OffsetsParams op{};
+    op.descs = &dev->head.desc;
+    op.hdrs = lp.hdrs;
+    op.lane_off = dev->lane_off;
+    op.payload_size = &dev->head.payload_size;
+    op.done = &dev->head.done;
+    op.n_tensors = 1;
+    lane_offsets_kernel<<<1, 256, 0, s>>>(op);
     CHK_CUDA(cudaGetLastError());
-    lane_scan_kernel<<<1, 256, 0, s>>>(&dev->desc, static_cast<LaneHeader*>(d_lane_headers), dev->payload_size,
-                                       dev->lane_off, 1u);
-    CHK_CUDA(cudaGetLastError());
-    tensor_scan_kernel<<<1, 1024, 0, s>>>(&dev->desc, dev->payload_size, dev->payload_off, 1u, nullptr);
-    CHK_CUDA(cudaGetLastError());
-    compact_kernel<<<32, 256, 0, s>>>(&dev->desc, static_cast<const LaneHeader*>(d_lane_headers), dev->lane_src,
-                                      dev->lane_off, base, static_cast<uint8_t*>(d_payload), 1u);
+    gather_lanes_kernel<<<(head.items[1] + 7) / 8, 256, 0, s>>>(lp.descs, dev->head.items, lp.hdrs, lp.lane_src, op.lane_off, base,
+                                                                static_cast<uint8_t*>(d_payload), 1u);
     CHK_CUDA(cudaGetLastError());
     struct {
-        unsigned long long size;
         TensorDesc desc;
+        unsigned long long size;
     } back;
-    CHK_CUDA(cudaMemcpyAsync(&back.size, dev->payload_size, 8, cudaMemcpyDeviceToHost, s));
-    CHK_CUDA(cudaMemcpyAsync(&back.desc, &dev->desc, sizeof(TensorDesc), cudaMemcpyDeviceToHost, s));
+    static_assert(offsetof(StaticHead, payload_size) == sizeof(TensorDesc), "read back in one copy");
+    CHK_CUDA(cudaMemcpyAsync(&back, &dev->head, sizeof(back), cudaMemcpyDeviceToHost, s));
     CHK_CUDA(cudaStreamSynchronize(s));
     *payload_size_out = back.size;
     if (is_raw_out) *is_raw_out = (back.desc.flags & kFlagRaw) ? 1 : 0;
