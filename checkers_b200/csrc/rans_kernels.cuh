@@ -423,17 +423,21 @@ __device__ __forceinline__ void encode_tensor(const TensorDesc& d, uint32_t ti, 
     __syncthreads();  // table and ring are reused by the next tensor
 }
 
-// One team (CTA of 64 threads) per tensor.  kInts = false is the build for
-// batches of float tensors only (two chains per thread, fewer registers, more
-// resident teams); the host picks the variant per batch.
-// Work is handed out through a ticket counter in the order given by `order`
-// (largest tensors first), so a persistent grid of resident teams drains the
-// batch without a ragged last wave.
+// One team (CTA of kTeam threads) per tensor.  kInts = false is the build for batches of float tensors only (one chain per
+// thread, fewer registers, more resident teams); the host picks the variant per batch.
+// Work is handed out through a ticket counter (zero at the start) in the order given by `order` (largest tensors first), so
+// a persistent grid of resident teams drains the batch without a ragged last wave.
 __device__ __forceinline__ uint32_t next_ticket(uint32_t* ticket, uint32_t* slot) {
     if (threadIdx.x == 0) *slot = atomicAdd(ticket, 1u);
     __syncthreads();
     return *slot;  // every thread reads it before the next barrier, which precedes the next write
 }
+// The same where a block's first item is its own number.  Blocks are spread over the SMs in the order of their numbers, so
+// the longest chains start on SMs of their own; when the first items are drawn too, two of them share an SM, and its
+// integer pipe, in every other call (a whole model, one chain of 524288 rows: encode 17.6, 20.4 or 26.1 ms, decode 21.7,
+// 23.9 or 28.3, now 17.6 and 21.6; 192 equal tensors: decode 0.240 -> 0.205 ms).  The decoders for batches of many small
+// tensors gain nothing by it and have no register to spare.
+__device__ __forceinline__ uint32_t later_ticket(uint32_t* ticket, uint32_t* slot) { return gridDim.x + next_ticket(ticket, slot); }
 
 template <bool kInts, bool kEscape>
 __global__ void __launch_bounds__(kTeam) rans_encode_kernel(const TensorDesc* __restrict__ descs,
@@ -781,15 +785,12 @@ __global__ void __launch_bounds__(kTeam, kInts ? CHK_LANES_INT_MINBLOCKS : CHK_L
     CHK_DYN_SMEM(smem);
     CHK_SHARED uint32_t s_ticket;
     const uint32_t zero_groups = (P.n_tensors + kTeam - 1) / kTeam;
-    for (;;) {
-        uint32_t tk = next_ticket(P.ticket, &s_ticket);
+    for (uint32_t tk = blockIdx.x; tk < zero_groups + P.n_tensors; tk = later_ticket(P.ticket, &s_ticket)) {
         if (tk < zero_groups) {
             zero_group(P, tk * kTeam, smem);
             continue;
         }
-        tk -= zero_groups;
-        if (tk >= P.n_tensors) break;
-        const uint32_t ti = P.order[tk];
+        const uint32_t ti = P.order[tk - zero_groups];
         const TensorDesc d = P.descs[ti];
         if (d.es == 4 && d.spe == 2)
             encode_tensor<1, 2, kEscape>(d, ti, P.tables, P.scratch, P.hdrs, P.lane_src, smem);
@@ -1182,9 +1183,7 @@ __global__ void __launch_bounds__(kTeam, kInts ? CHK_ENC_INT_MINBLOCKS : CHK_ENC
     CHK_DYN_SMEM(smem);
     CHK_SHARED uint32_t s_ticket;
     uint8_t* const slot = P.scratch + (unsigned long long)blockIdx.x * P.slot_bytes;
-    for (;;) {
-        const uint32_t tk = next_ticket(P.ticket, &s_ticket);
-        if (tk >= P.n_tensors) break;
+    for (uint32_t tk = blockIdx.x; tk < P.n_tensors; tk = later_ticket(P.ticket, &s_ticket)) {
         const uint32_t ti = P.order[tk];
         const uint32_t es = P.descs[ti].es, spe = P.descs[ti].spe;
         if (es == 4 && spe == 2)
@@ -2263,9 +2262,7 @@ __global__ void __launch_bounds__(SplitSmem<kKind>::kChains + kSplitHelpers, kKi
     CHK_DYN_SMEM(smem);
     CHK_SHARED uint32_t s_ticket;
     constexpr uint32_t kThreads = SplitSmem<kKind>::kChains + kSplitHelpers;
-    for (;;) {
-        const uint32_t tk = next_ticket(P.ticket, &s_ticket);
-        if (tk >= P.n_units) break;
+    for (uint32_t tk = blockIdx.x; tk < P.n_units; tk = later_ticket(P.ticket, &s_ticket)) {
         const uint32_t unit = P.units[tk];
         if (kKind == 0) {
             const TensorDesc d = P.descs[unit & 0x7FFFFFFFu];
