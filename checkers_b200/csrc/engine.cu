@@ -9,11 +9,12 @@
 //   split_hist_kernel         low bytes -> final .mant data layout, histograms; in a few pieces
 //   normalize_tables_kernel   frequency tables and encode entries of a piece, on the device,
 //   zero_chain_kernel         while the next piece is counted (a second stream)
-//   rans_encode_fused_kernel  one persistent grid of 64-thread teams, one tensor at a time each,
+//   rans_encode_fused_kernel  one persistent grid of 128-thread teams, one tensor at a time each,
 //                             largest first: lanes, lane offsets, passthrough rule, headers and
 //                             the gather of the lanes into a payload heap
-// with ONE host synchronisation per checkpoint; the payload of each tensor is then copied
-// to its place in the .ansc image (file order) and the other two images by a large copy each.
+// or, for batches whose lane regions fit the scratch of the resident teams, lanes, offsets and gather
+// as launches of their own (rans_lanes_kernel and the two after it), with ONE host synchronisation per
+// checkpoint; the data section then crosses to the host in file order in one copy, and so do the other images.
 #include <cuda_runtime.h>
 
 #include <chrono>

@@ -434,7 +434,7 @@ __device__ __forceinline__ uint32_t next_ticket(uint32_t* ticket, uint32_t* slot
 }
 // The same where a block's first item is its own number.  Blocks are spread over the SMs in the order of their numbers, so
 // the longest chains start on SMs of their own; when the first items are drawn too, two of them share an SM, and its
-// integer pipe, in every other call (a whole model, one chain of 524288 rows: encode 17.6, 20.4 or 26.1 ms, decode 21.7,
+// integer pipe, in every other call (a whole model, chains of 512000 rows: encode 17.6, 20.4 or 26.1 ms, decode 21.7,
 // 23.9 or 28.3, now 17.6 and 21.6; 192 equal tensors: decode 0.240 -> 0.205 ms).  The decoders for batches of many small
 // tensors gain nothing by it and have no register to spare.
 __device__ __forceinline__ uint32_t later_ticket(uint32_t* ticket, uint32_t* slot) { return gridDim.x + next_ticket(ticket, slot); }
