@@ -2080,7 +2080,7 @@ __device__ __forceinline__ void split_unit(const SplitParams& P, uint32_t unit, 
     constexpr int kLow = kKind == 2 ? 16 : kKind == 1 ? 4 : 8;
     const uint8_t* low_col = nullptr;
     uint8_t* dst_col = nullptr;
-    bool low_ok = false, dst_ok = false;
+    bool low_ok = false, dst_ok = false, dst_even = false;
     uint32_t row0 = 0;
     if (!stepping) {
         if (floats) {
@@ -2102,6 +2102,7 @@ __device__ __forceinline__ void split_unit(const SplitParams& P, uint32_t unit, 
             low_ok = kKind == 0 || (reinterpret_cast<uintptr_t>(low_col) & 3) == 0;
             dst_ok = (reinterpret_cast<uintptr_t>(dst_col) & (kKind == 1 ? 7 : 3)) == 0;
         }
+        dst_even = (reinterpret_cast<uintptr_t>(dst_col) & 1) == 0;
     }
     uint32_t low[kLow];
     auto load_low = [&](uint32_t row, auto fast) {  // of rows row + row0 ...
@@ -2123,6 +2124,9 @@ __device__ __forceinline__ void split_unit(const SplitParams& P, uint32_t unit, 
     auto put32 = [&](uint8_t* p, uint32_t w, auto fast) {
         if (decltype(fast)::value) {
             *reinterpret_cast<uint32_t*>(p) = w;
+        } else if (dst_even) {
+            reinterpret_cast<uint16_t*>(p)[0] = (uint16_t)w;
+            reinterpret_cast<uint16_t*>(p)[1] = (uint16_t)(w >> 16);
         } else {
 #pragma unroll
             for (int b = 0; b < 4; ++b) p[b] = (uint8_t)(w >> (8 * b));
@@ -2167,11 +2171,8 @@ __device__ __forceinline__ void split_unit(const SplitParams& P, uint32_t unit, 
                     if (decltype(fast)::value) {
                         *reinterpret_cast<uint2*>(p) = make_uint2(e01, e23);
                     } else {
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            p[b] = (uint8_t)(e01 >> (8 * b));
-                            p[4 + b] = (uint8_t)(e23 >> (8 * b));
-                        }
+                        put32(p, e01, fast);
+                        put32(p + 4, e23, fast);
                     }
                 }
             }
@@ -2216,7 +2217,7 @@ __device__ __forceinline__ void split_unit(const SplitParams& P, uint32_t unit, 
                 g.dst[at * 4 + 2 + plane_of(tid)] = (uint8_t)v;
         }
     } else {
-        auto loop = [&](auto fast) {
+        auto loop = [&](auto fast_low, auto fast_dst) {
             uint4 v[kKind == 2 ? 4 : 2] = {};  // blocks on their way
             uint32_t take[kKind == 2 ? 2 : 1] = {};
             for (uint32_t p = 0; p < periods; ++p) {
@@ -2227,13 +2228,19 @@ __device__ __forceinline__ void split_unit(const SplitParams& P, uint32_t unit, 
                     take[k] = p > 0 && f.gp < f.gend && f.loaded - (sm->pos[(p - 1) & 1][h + k * kSplitHelpers] >> 3) <= 96u;
                     split_load(take[k], f.gp, f.gp + 32 < f.gend, v[2 * k], v[2 * k + 1]);
                 }
-                if (p > 0) write_rows((p - 1) * 16, sm->out[(p - 1) & 1], fast);
-                load_low(p * 16, fast);
+                if (p > 0) write_rows((p - 1) * 16, sm->out[(p - 1) & 1], fast_dst);
+                load_low(p * 16, fast_low);
                 period_barrier();
             }
-            if (periods) write_rows((periods - 1) * 16, sm->out[(periods - 1) & 1], fast);
+            if (periods) write_rows((periods - 1) * 16, sm->out[(periods - 1) & 1], fast_dst);
         };
-        if (low_ok && dst_ok) loop(std::true_type{}); else loop(std::false_type{});
+        // Low bytes start at any address once a tensor before had an odd number of elements; the tensors themselves then
+        // still start on an element.  (50 M elements of Adam state in odd slices: 0.90 ms, 1.10 with one choice for both.)
+        if (dst_ok) {
+            if (low_ok) loop(std::true_type{}, std::true_type{}); else loop(std::false_type{}, std::true_type{});
+        } else {
+            if (low_ok) loop(std::true_type{}, std::false_type{}); else loop(std::false_type{}, std::false_type{});
+        }
         if (kKind != 0 || floats) {  // low bytes of the rows that are left
             const uint32_t per = kKind == 0 ? d.spe : (uint32_t)kKind;  // low bytes of an element
             const uint32_t es = kKind == 0 ? d.es : 2u * (uint32_t)kKind;
