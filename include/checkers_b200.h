@@ -88,7 +88,7 @@ int chk_tensor_count(chk_context* ctx, uint64_t* count);
  * "allow_undecodable" (0/1; see chk_compress_and_save), "verify_zero_lanes" (0/1;
  * decode also checks the lanes that only carry zeroed low bytes),
  * "workspace_bytes" (bound on the encode scratch, as in chk_context_create_ex),
- * "segments" (1..8, default 4: launches the counting of a batch of 512 tensors or
+ * "segments" (1..8, default 4: launches the counting of a large batch, 512 tensors or
  * more is cut into, so that the tables of one piece are built while the next is
  * counted), "encode_teams_per_sm" / "decode_teams_per_sm" (default 0 = as many as
  * fit: cap on the resident teams per SM), "decode_zero_skip" (0/1; float tensors
@@ -192,7 +192,7 @@ int chk_normalize_histogram(const uint32_t hist[256], int ensure_full_alphabet, 
 
 /* ---- timing: the reference's [TIMING] / per-tensor ms fields -------------
  * Keys: split_hist_ms (counting), table_ms (what of the table building the counting did not hide),
- * encode_ms (lanes, offsets and gather: one kernel), compress_device_ms, encode_teams, workspace_mb,
+ * encode_ms (lanes, offsets and gather), compress_device_ms, encode_teams, workspace_mb,
  * d2h_ms, io_ms, compress_total_ms, h2d_ms, decode_ms, decompress_total_ms,
  * analyze_stats_ms, analyze_cluster_ms.  Device spans are CUDA-event times. */
 int chk_get_timing(chk_context* ctx, const char* key, double* ms);
